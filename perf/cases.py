@@ -312,3 +312,77 @@ def tolerance(case):
     if case["kind"] == "forward":
         return {"rel": {"f16": 4e-3, "bf16": 3e-2, "f32": 1e-4}[d]}
     return {"rel": {"f16": 1e-3, "bf16": 7e-3, "f32": 1.5e-5}[d]}
+
+
+def exact(case, seed):
+    """What ``run`` returns for these inputs in 64-bit arithmetic, written with plain torch."""
+    c = case
+    kind = c["kind"]
+    if kind == "forward":
+        return _exact_forward(c, seed)
+    s = prepare(case, seed)
+    if kind == "gemm":
+        A, B = s["A"].double(), s["B"].double()
+        y = c["alpha"] * ((A.t() if c["ta"] else A) @ (B.t() if c["tb"] else B))
+        return y + c["beta"] * s["C"].double() if c["beta"] != 0 else y
+    if kind == "batched":
+        return torch.bmm(s["A"].double(), (s["B"].transpose(1, 2) if c["tb"] else s["B"]).double())
+    if kind == "conv":
+        return _conv64(s["X"].double(), s["W"].double(), s["b"].double(), c["stride"], c["pad"], c["dilation"], c["group"],
+                       s["R"], c["relu"])
+    T, B = s["T"].double(), s["B"].double()
+    if c["routine"] == "syrk":
+        full = B @ B.t()
+        return torch.triu(full) if c["upper"] else torch.tril(full)
+    part = torch.triu(T) if c["upper"] else torch.tril(T)
+    if c["routine"] == "symm":
+        part = part + part.t() - torch.diag(part.diagonal())
+        return part @ B if c["left"] else B @ part
+    upper = c["upper"] != c["trans"]
+    part = part.t() if c["trans"] else part
+    if c["routine"] == "trmm":
+        return part @ B if c["left"] else B @ part
+    return torch.linalg.solve_triangular(part, B, upper=upper, left=c["left"])
+
+
+def _conv64(x, w, b, stride, pad, dilation, group, residual, relu):
+    """One filter tap after the other: a strided window of the bordered images times its weights."""
+    n, cin, h, wd = x.shape
+    cout, cg, kh, kw = w.shape
+    oh = (h + 2 * pad - dilation * (kh - 1) - 1) // stride + 1
+    ow = (wd + 2 * pad - dilation * (kw - 1) - 1) // stride + 1
+    xp = torch.nn.functional.pad(x, (pad, pad, pad, pad)) if pad else x
+    y = b.view(1, group, cout // group, 1).expand(n, group, cout // group, oh * ow).contiguous()
+    wg = w.view(group, cout // group, cg, kh, kw)
+    for i in range(kh):
+        for j in range(kw):
+            win = xp[:, :, i * dilation:i * dilation + (oh - 1) * stride + 1:stride,
+                     j * dilation:j * dilation + (ow - 1) * stride + 1:stride]
+            y += torch.matmul(wg[:, :, :, i, j], win.reshape(n, group, cg, oh * ow))
+    y = y.view(n, cout, oh, ow)
+    if residual is not None:
+        y += residual.double()
+    return y.clamp_(min=0) if relu else y
+
+
+def _exact_forward(c, seed):
+    """ResNet-50 on the parameters of `_resnet50`, as the case's type holds them."""
+    t = _TYPES[c["dtype"]]
+    graph = _resnet50(c["batch"], c["size"], seed)
+    par = {v.name: torch.from_numpy(v.initializer).cuda().to(t).double() for v in graph.inputs if v.has_initializer()}
+
+    def conv(x, name, stride, pad, residual=None, relu=True):
+        return _conv64(x, par[name + ".W"], par[name + ".B"], stride, pad, 1, 1, residual, relu)
+
+    images = _randn(seed + 1000, (c["batch"], 3, c["size"], c["size"]), c["dtype"])
+    logits = []
+    for part in images.split(16):
+        x = conv(part.double(), "conv1", 2, 3)
+        x = torch.nn.functional.max_pool2d(x, 3, 2, 1)
+        for stage, (blocks, _, stride) in enumerate(_STAGES):
+            for b in range(blocks):
+                nm, st = "s%db%d" % (stage + 1, b), stride if b == 0 else 1
+                a = conv(conv(x, nm + ".c1", st, 0), nm + ".c2", 1, 1)
+                x = conv(a, nm + ".c3", 1, 0, conv(x, nm + ".down", st, 0, relu=False) if b == 0 else x)
+        logits.append(x.mean((2, 3)) @ par["fc.W"].t() + par["fc.B"])
+    return torch.cat(logits)
