@@ -1279,6 +1279,46 @@ int l3_expand_any(int fmt, void* dst, const void* src, size_t ld, size_t n, bool
 
 namespace {
 
+// Systems per CTA of a triangular solve: the fewest that let all CTAs run at once (a step of the chain takes
+// warp 0 as long for 4 systems as for 24, the other warps' part grows with them), 24 when that is not to be had.
+template <typename T, bool EQC, int C>
+int trsm_launch(const void* base, long long se, long long sv, bool unit, size_t q, void* b, long long bu, long long bs,
+                size_t nsys, float alpha, cudaStream_t s) {
+    const size_t smem = trsm_smem_bytes(static_cast<int>(q), C, EQC);
+    auto kernel = l3_trsm_kernel<T, EQC, C>;
+    CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    kernel<<<static_cast<unsigned>((nsys + C - 1) / C), kTrsmThreads, smem, s>>>(
+        static_cast<const T*>(base), se, sv, unit ? 1 : 0, static_cast<int>(q), static_cast<T*>(b), bu, bs,
+        static_cast<int>(nsys), alpha);
+    g_launches.fetch_add(1);
+    CUDA_TRY(cudaGetLastError());
+    return kSuccess;
+}
+
+template <typename T, bool EQC>
+int trsm_columns(const void* base, long long se, long long sv, bool unit, size_t q, void* b, long long bu, long long bs,
+                 size_t nsys, float alpha, cudaStream_t s) {
+    if (nsys <= 4 * 148) return trsm_launch<T, EQC, 4>(base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
+    if (nsys <= 8 * 148) return trsm_launch<T, EQC, 8>(base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
+    if (nsys <= 16 * 148) return trsm_launch<T, EQC, 16>(base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
+    return trsm_launch<T, EQC, 24>(base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
+}
+
+template <typename T>
+int trsm_any(bool eqc, const void* base, long long se, long long sv, bool unit, size_t q, void* b, long long bu,
+             long long bs, size_t nsys, float alpha, cudaStream_t s) {
+    return eqc ? trsm_columns<T, true>(base, se, sv, unit, q, b, bu, bs, nsys, alpha, s)
+               : trsm_columns<T, false>(base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
+}
+
+// one diagonal block (order q <= kTrsmOrder) of a triangular solve; arguments as of l3_trsm_kernel
+int trsm_block(int fmt, const void* base, long long se, long long sv, bool eqc, bool unit, size_t q, void* b,
+               long long bu, long long bs, size_t nsys, float alpha, cudaStream_t s) {
+    if (fmt == FMT_F32) return trsm_any<float>(eqc, base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
+    if (fmt == FMT_F16) return trsm_any<__half>(eqc, base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
+    return trsm_any<__nv_bfloat16>(eqc, base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
+}
+
 // common argument rules of trmm / trsm; on success the call is in row-major form
 int tri_args(int dtype, int& fmt, int& es, int layout, int& side, int& triangle, int a_transpose, int diagonal,
              size_t& m, size_t& n, const void* alpha, const void* a, size_t a_ld, const void* b, size_t b_ld) {
@@ -2366,7 +2406,8 @@ int dlf_b200_trsm(int dtype, int layout, int side, int triangle, int a_transpose
     char* B = static_cast<char*>(b);
     auto a_at = [&](size_t r, size_t c) { return A + (r * a_ld + c) * es; };
     auto b_at = [&](size_t r, size_t c) { return B + (r * b_ld + c) * es; };
-    if (al != 1.0f) {
+    // one block: alpha goes in with its right-hand sides; more: the updates need all of B scaled
+    if (al != 1.0f && (side == kLeft ? m : n) > kTrsmOrder) {
         const unsigned grid = l3_grid(static_cast<long long>(m) * n);
         if (fmt == FMT_F32) l3_scale_kernel<float><<<grid, 256, 0, s>>>(reinterpret_cast<float*>(B), static_cast<long long>(b_ld), static_cast<int>(m), static_cast<int>(n), al);
         else if (fmt == FMT_F16) l3_scale_kernel<__half><<<grid, 256, 0, s>>>(reinterpret_cast<__half*>(B), static_cast<long long>(b_ld), static_cast<int>(m), static_cast<int>(n), al);
@@ -2374,27 +2415,27 @@ int dlf_b200_trsm(int dtype, int layout, int side, int triangle, int a_transpose
         g_launches.fetch_add(1);
         CUDA_TRY(cudaGetLastError());
     }
-    auto diag_solve = [&](size_t d0, size_t nb, char* bblk, size_t nsys) -> int {
-        const unsigned grid = static_cast<unsigned>((nsys + kTrsmThreads - 1) / kTrsmThreads);
-        const int rs = side == kRight ? 1 : 0;
-        if (fmt == FMT_F32)
-            l3_trsm_diag_kernel<float><<<grid, kTrsmThreads, 0, s>>>(reinterpret_cast<const float*>(a_at(d0, d0)), static_cast<long long>(a_ld), trans, lower, diagonal == kUnit, rs, static_cast<int>(nb), reinterpret_cast<float*>(bblk), static_cast<long long>(b_ld), static_cast<int>(nsys));
-        else if (fmt == FMT_F16)
-            l3_trsm_diag_kernel<__half><<<grid, kTrsmThreads, 0, s>>>(reinterpret_cast<const __half*>(a_at(d0, d0)), static_cast<long long>(a_ld), trans, lower, diagonal == kUnit, rs, static_cast<int>(nb), reinterpret_cast<__half*>(bblk), static_cast<long long>(b_ld), static_cast<int>(nsys));
-        else
-            l3_trsm_diag_kernel<__nv_bfloat16><<<grid, kTrsmThreads, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(a_at(d0, d0)), static_cast<long long>(a_ld), trans, lower, diagonal == kUnit, rs, static_cast<int>(nb), reinterpret_cast<__nv_bfloat16*>(bblk), static_cast<long long>(b_ld), static_cast<int>(nsys));
-        g_launches.fetch_add(1);
-        CUDA_TRY(cudaGetLastError());
-        return kSuccess;
+    // order of the blocks: as few as kTrsmOrder allows, of about equal order
+    const size_t order = side == kLeft ? m : n, nsys = side == kLeft ? n : m;
+    const size_t parts = (order + kTrsmOrder - 1) / kTrsmOrder;
+    const size_t block = ((order + parts - 1) / parts + 31) / 32 * 32;
+    auto diag_solve = [&](size_t d0, size_t nb, float scale) -> int {
+        const bool forward = side == kLeft ? op_lower : !op_lower;
+        const long long d1 = static_cast<long long>(forward ? d0 : d0 + nb - 1), dir = forward ? 1 : -1;
+        const bool eqc = (side == kRight) != trans;
+        const long long se = dir * (eqc ? 1 : static_cast<long long>(a_ld)), sv = dir * (eqc ? static_cast<long long>(a_ld) : 1);
+        const long long bu = side == kLeft ? dir * static_cast<long long>(b_ld) : dir, bs = side == kLeft ? 1 : static_cast<long long>(b_ld);
+        char* first = side == kLeft ? b_at(d1, 0) : b_at(0, d1);
+        return trsm_block(fmt, a_at(d1, d1), se, sv, eqc, diagonal == kUnit, nb, first, bu, bs, nsys, scale, s);
     };
     const int N = DLF_B200_NO_TRANS, T = DLF_B200_TRANS;
     if (side == kLeft) {
         // op(T) X = B: row blocks of B, top to bottom when op(T) is lower, else bottom to top;
         // every block first loses the contribution of the rows already solved (a GEMM)
-        const size_t blocks = (m + kTrsmBlock - 1) / kTrsmBlock;
+        const size_t blocks = (m + block - 1) / block;
         for (size_t bi = 0; bi < blocks; ++bi) {
             const size_t blk = op_lower ? bi : blocks - 1 - bi;
-            const size_t i0 = blk * kTrsmBlock, i1 = std::min<size_t>(m, i0 + kTrsmBlock), ib = i1 - i0;
+            const size_t i0 = blk * block, i1 = std::min<size_t>(m, i0 + block), ib = i1 - i0;
             if (op_lower && i0 > 0) {
                 rc = trans ? rm_gemm(fmt, T, N, ib, n, i0, -1.0f, a_at(0, i0), a_ld, b_at(0, 0), b_ld, 1.0f, b_at(i0, 0), b_ld, stream)
                            : rm_gemm(fmt, N, N, ib, n, i0, -1.0f, a_at(i0, 0), a_ld, b_at(0, 0), b_ld, 1.0f, b_at(i0, 0), b_ld, stream);
@@ -2403,15 +2444,15 @@ int dlf_b200_trsm(int dtype, int layout, int side, int triangle, int a_transpose
                            : rm_gemm(fmt, N, N, ib, n, m - i1, -1.0f, a_at(i0, i1), a_ld, b_at(i1, 0), b_ld, 1.0f, b_at(i0, 0), b_ld, stream);
             }
             if (rc != kSuccess) return rc;
-            rc = diag_solve(i0, ib, b_at(i0, 0), n);
+            rc = diag_solve(i0, ib, parts > 1 ? 1.0f : al);
             if (rc != kSuccess) return rc;
         }
     } else {
         // X op(T) = B: column blocks of B, left to right when op(T) is upper, else right to left
-        const size_t blocks = (n + kTrsmBlock - 1) / kTrsmBlock;
+        const size_t blocks = (n + block - 1) / block;
         for (size_t bi = 0; bi < blocks; ++bi) {
             const size_t blk = op_lower ? blocks - 1 - bi : bi;
-            const size_t j0 = blk * kTrsmBlock, j1 = std::min<size_t>(n, j0 + kTrsmBlock), jb = j1 - j0;
+            const size_t j0 = blk * block, j1 = std::min<size_t>(n, j0 + block), jb = j1 - j0;
             if (!op_lower && j0 > 0) {
                 rc = trans ? rm_gemm(fmt, N, T, m, jb, j0, -1.0f, b_at(0, 0), b_ld, a_at(j0, 0), a_ld, 1.0f, b_at(0, j0), b_ld, stream)
                            : rm_gemm(fmt, N, N, m, jb, j0, -1.0f, b_at(0, 0), b_ld, a_at(0, j0), a_ld, 1.0f, b_at(0, j0), b_ld, stream);
@@ -2420,7 +2461,7 @@ int dlf_b200_trsm(int dtype, int layout, int side, int triangle, int a_transpose
                            : rm_gemm(fmt, N, N, m, jb, n - j1, -1.0f, b_at(0, j1), b_ld, a_at(j1, j0), a_ld, 1.0f, b_at(0, j0), b_ld, stream);
             }
             if (rc != kSuccess) return rc;
-            rc = diag_solve(j0, jb, b_at(0, j0), m);
+            rc = diag_solve(j0, jb, parts > 1 ? 1.0f : al);
             if (rc != kSuccess) return rc;
         }
     }
