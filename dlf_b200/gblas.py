@@ -10,6 +10,7 @@ reference's ``StatusCode`` value. Every call goes through the C-ABI of libdlf_b2
 """
 import ctypes
 import enum
+import math
 import threading
 
 import torch
@@ -86,8 +87,18 @@ def precision_of(buf):
         raise BLASError(StatusCode.kNotImplemented)
 
 
+# the scalars nearly every call passes, in each storage type (never written to)
+_ONE = {torch.float16: ctypes.c_uint16(0x3C00), torch.bfloat16: ctypes.c_uint16(0x3F80), torch.float32: ctypes.c_float(1.0)}
+_ZERO = {torch.float16: ctypes.c_uint16(0), torch.bfloat16: ctypes.c_uint16(0), torch.float32: ctypes.c_float(0.0)}
+
+
 def _scalar(value, dtype):
     """Packs a host scalar in the storage type T, as the reference passes `const T alpha`."""
+    if type(value) is int or type(value) is float:
+        if value == 1:
+            return _ONE[dtype]
+        if value == 0 and math.copysign(1.0, value) > 0:
+            return _ZERO[dtype]
     t = torch.tensor([value], dtype=dtype)
     if dtype == torch.float32:
         return ctypes.c_float(float(t.item()))
@@ -109,6 +120,11 @@ def _ptr(buf, offset=0):
 def _stream(queue):
     s = queue if queue is not None else torch.cuda.current_stream()
     return s, ctypes.c_void_p(s.cuda_stream)
+
+
+def _raw_stream(queue):
+    """The stream of a call as an integer handle, without building a Stream object for it."""
+    return queue.cuda_stream if queue is not None else torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 _GEMM_WORKSPACES = {}
@@ -144,15 +160,16 @@ def _caller_scratch(device, nbytes):
     return buf
 
 
-def _gemm_workspace(device, stream, nbytes):
+def _gemm_workspace(device, queue, handle, nbytes):
     """One scratch buffer per (device, stream), grown on demand; calls on a stream are ordered, so
-    they can share it."""
+    they can share it. `handle` is the stream's handle, `queue` the stream (None = the current one)."""
     own = _caller_scratch(device, nbytes)
     if own is not None:
         return own
-    key = (device.index, stream.cuda_stream)
+    key = (device.index, handle)
     buf = _GEMM_WORKSPACES.get(key)
     if buf is None or buf.numel() < nbytes:
+        stream = queue if queue is not None else torch.cuda.current_stream()
         if buf is not None:
             buf.record_stream(stream)
         buf = torch.empty(int(nbytes), dtype=torch.uint8, device=device)
@@ -200,28 +217,62 @@ def _validate(layout, ta, tb, m, n, k, a, a_off, a_ld, b, b_off, b_ld, c, c_off,
                      StatusCode.kInsufficientMemoryC)
 
 
+class _Operand:
+    """A matrix operand as the library sees it: address of its first element, and how many elements
+    its buffer holds beyond what a call may address (`numel`, counted from the buffer's start)."""
+
+    __slots__ = ("dtype", "device", "is_cuda", "address", "offset", "count")
+
+    def __init__(self, tensor, storage_elements, offset):
+        self.dtype = tensor.dtype
+        self.device = tensor.device
+        self.is_cuda = tensor.is_cuda
+        self.count = storage_elements
+        self.offset = offset
+        self.address = tensor.data_ptr()
+
+    def numel(self):
+        return self.count
+
+
+def _view_operand(t):
+    """The operand that starts at a (strided) tensor's first element, inside its whole storage."""
+    return _Operand(t, t.untyped_storage().nbytes() // t.element_size(), t.storage_offset())
+
+
+def _buffer_operand(buf, offset):
+    op = _Operand(buf, buf.numel(), offset)
+    op.address += int(offset) * buf.element_size()
+    return op
+
+
 def gemm(layout, a_transpose, b_transpose, m, n, k, alpha, a_buffer, a_offset, a_ld, b_buffer,
          b_offset, b_ld, beta, c_buffer, c_offset, c_ld, queue=None, event=None):
     """C = alpha*op(A)*op(B) + beta*C  (gpgpu::blas::gemm, gblas.h:496-504)."""
-    prec = precision_of(c_buffer)
-    if a_buffer.dtype != c_buffer.dtype or b_buffer.dtype != c_buffer.dtype:
+    _gemm(layout, a_transpose, b_transpose, m, n, k, alpha, _buffer_operand(a_buffer, a_offset), a_ld,
+          _buffer_operand(b_buffer, b_offset), b_ld, beta, _buffer_operand(c_buffer, c_offset), c_ld, queue, event)
+
+
+def _gemm(layout, a_transpose, b_transpose, m, n, k, alpha, a, a_ld, b, b_ld, beta, c, c_ld, queue=None, event=None):
+    prec = precision_of(c)
+    if a.dtype != c.dtype or b.dtype != c.dtype:
         raise BLASError(StatusCode.kInvalidValue)
-    _validate(layout, a_transpose, b_transpose, m, n, k, a_buffer, [a_offset], a_ld, b_buffer,
-              [b_offset], b_ld, c_buffer, [c_offset], c_ld)
-    al, be = _scalar(alpha, c_buffer.dtype), _scalar(beta, c_buffer.dtype)
-    s, sp = _stream(queue)
+    _validate(layout, a_transpose, b_transpose, m, n, k, a, (a.offset,), a_ld, b, (b.offset,), b_ld, c, (c.offset,), c_ld)
+    al, be = _scalar(alpha, c.dtype), _scalar(beta, c.dtype)
+    if not (a.is_cuda and b.is_cuda and c.is_cuda):
+        raise BLASError(StatusCode.kInvalidMatrixA)
+    L = lib()
+    handle = _raw_stream(queue)
     # scratch for a K-split of products with few output tiles (the reference's Xgemm takes its
     # temporaries from the context's pool, routines/level3/xgemm.cpp:107-223); 0 bytes = not useful
-    need = lib().dlf_b200_gemm_workspace_bytes(int(prec), m, n, k)
-    ws = _gemm_workspace(c_buffer.device, s, need) if need else None
+    need = L.dlf_b200_gemm_workspace_bytes(int(prec), m, n, k)
+    ws = _gemm_workspace(c.device, queue, handle, need) if need else None
     if event is not None:
+        s = queue if queue is not None else torch.cuda.current_stream()
         event.start.record(s)
-    rc = lib().dlf_b200_gemm_ex(int(prec), int(layout), int(a_transpose), int(b_transpose), m, n, k,
-                                ctypes.byref(al), _ptr(a_buffer, a_offset), a_ld,
-                                _ptr(b_buffer, b_offset), b_ld, ctypes.byref(be),
-                                _ptr(c_buffer, c_offset), c_ld,
-                                ctypes.c_void_p(ws.data_ptr()) if ws is not None else None,
-                                ws.numel() if ws is not None else 0, sp)
+    rc = L.dlf_b200_gemm_ex(int(prec), int(layout), int(a_transpose), int(b_transpose), m, n, k, ctypes.byref(al), a.address, a_ld,
+                            b.address, b_ld, ctypes.byref(be), c.address, c_ld,
+                            ws.data_ptr() if ws is not None else None, ws.numel() if ws is not None else 0, handle)
     if event is not None:
         event.end.record(s)
     _check(rc)
@@ -231,23 +282,31 @@ def gemmStridedBatched(layout, a_transpose, b_transpose, m, n, k, alpha, a_buffe
                        a_stride, b_buffer, b_offset, b_ld, b_stride, beta, c_buffer, c_offset,
                        c_ld, c_stride, batch_count, queue=None, event=None):
     """gpgpu::blas::gemmStridedBatched (gblas.h:673-683); a stride of 0 shares an operand."""
-    prec = precision_of(c_buffer)
-    if a_buffer.dtype != c_buffer.dtype or b_buffer.dtype != c_buffer.dtype:
+    _gemm_strided(layout, a_transpose, b_transpose, m, n, k, alpha, _buffer_operand(a_buffer, a_offset), a_ld, a_stride,
+                  _buffer_operand(b_buffer, b_offset), b_ld, b_stride, beta, _buffer_operand(c_buffer, c_offset), c_ld,
+                  c_stride, batch_count, queue, event)
+
+
+def _gemm_strided(layout, a_transpose, b_transpose, m, n, k, alpha, a, a_ld, a_stride, b, b_ld, b_stride, beta, c, c_ld,
+                  c_stride, batch_count, queue=None, event=None):
+    prec = precision_of(c)
+    if a.dtype != c.dtype or b.dtype != c.dtype:
         raise BLASError(StatusCode.kInvalidValue)
     if batch_count < 1:
         raise BLASError(StatusCode.kInvalidBatchCount)
     last = batch_count - 1
-    _validate(layout, a_transpose, b_transpose, m, n, k, a_buffer, [a_offset + last * a_stride],
-              a_ld, b_buffer, [b_offset + last * b_stride], b_ld, c_buffer,
-              [c_offset + last * c_stride], c_ld)
-    al, be = _scalar(alpha, c_buffer.dtype), _scalar(beta, c_buffer.dtype)
-    s, sp = _stream(queue)
+    _validate(layout, a_transpose, b_transpose, m, n, k, a, (a.offset + last * a_stride,), a_ld, b,
+              (b.offset + last * b_stride,), b_ld, c, (c.offset + last * c_stride,), c_ld)
+    al, be = _scalar(alpha, c.dtype), _scalar(beta, c.dtype)
+    if not (a.is_cuda and b.is_cuda and c.is_cuda):
+        raise BLASError(StatusCode.kInvalidMatrixA)
+    handle = _raw_stream(queue)
     if event is not None:
+        s = queue if queue is not None else torch.cuda.current_stream()
         event.start.record(s)
     rc = lib().dlf_b200_gemm_strided_batched(
-        int(prec), int(layout), int(a_transpose), int(b_transpose), m, n, k, ctypes.byref(al),
-        _ptr(a_buffer, a_offset), a_ld, a_stride, _ptr(b_buffer, b_offset), b_ld, b_stride,
-        ctypes.byref(be), _ptr(c_buffer, c_offset), c_ld, c_stride, batch_count, sp)
+        int(prec), int(layout), int(a_transpose), int(b_transpose), m, n, k, ctypes.byref(al), a.address, a_ld, a_stride, b.address, b_ld,
+        b_stride, ctypes.byref(be), c.address, c_ld, c_stride, batch_count, handle)
     if event is not None:
         event.end.record(s)
     _check(rc)

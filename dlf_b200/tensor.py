@@ -53,11 +53,18 @@ def gemm(transA, transB, alpha, A, B, beta, C, Y=None, backend=None):
             Y.copy_(C.expand(m, n))
         except RuntimeError:
             raise ShapeError("gemm: C is not broadcastable to {m, n}")
-    be.gemm(Layout.RowMajor, transA, transB, m, n, k, alpha,
-            _flat(A), A.storage_offset(), max(A.stride(0), 1),
-            _flat(B), B.storage_offset(), max(B.stride(0), 1), beta,
-            _flat(Y), Y.storage_offset(), max(Y.stride(0), 1))
+    _gemm(be, transA, transB, m, n, k, alpha, A, max(A.stride(0), 1), B, max(B.stride(0), 1), beta, Y, max(Y.stride(0), 1))
     return Y
+
+
+def _gemm(be, transA, transB, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc):
+    """be.gemm on views; the library's own mirror takes their addresses without flat views of the storages."""
+    if be is _gblas:
+        be._gemm(Layout.RowMajor, transA, transB, m, n, k, alpha, be._view_operand(A), lda, be._view_operand(B), ldb, beta,
+                 be._view_operand(C), ldc)
+    else:
+        be.gemm(Layout.RowMajor, transA, transB, m, n, k, alpha, _flat(A), A.storage_offset(), lda,
+                _flat(B), B.storage_offset(), ldb, beta, _flat(C), C.storage_offset(), ldc)
 
 
 def _is_contiguous_strides(shape, strides):
@@ -121,12 +128,14 @@ def _broadcast(A, B):
     p, n = B.shape[-2:]
     if k != p:
         raise ShapeError("matmul: Incompatible dimensions for matrix multiplication")
-    try:
-        prefix = torch.broadcast_shapes(tuple(A.shape[:-2]), tuple(B.shape[:-2]))
-    except RuntimeError:
-        raise ShapeError("matmul: batch dimensions are not broadcastable")
-    A = A.expand(*prefix, m, k)
-    B = B.expand(*prefix, k, n)
+    prefix = A.shape[:-2]
+    if B.shape[:-2] != prefix:
+        try:
+            prefix = torch.broadcast_shapes(tuple(prefix), tuple(B.shape[:-2]))
+        except RuntimeError:
+            raise ShapeError("matmul: batch dimensions are not broadcastable")
+        A = A.expand(*prefix, m, k)
+        B = B.expand(*prefix, k, n)
     batch = 1
     for e in prefix:
         batch *= e
@@ -214,31 +223,33 @@ def matmul(A, B, C=None, alpha=1, beta=0, backend=None, trace=None):
     if transB == Transpose.Trans:
         ldb = max(ldb, k)
 
-    fa, fb, fc = _flat(vA), _flat(vB), _flat(vC)
-    sa, sb, sc = list(vA.stride()), list(vB.stride()), list(vC.stride())
+    sa, sb, sc = vA.stride(), vB.stride(), vC.stride()
     if batch == 1:
         # the reference sends m == n == 1 to gblas::dot and n == 1 to gblas::gemv; both are the
         # same contraction, served here by the gemm entry point
         if trace is not None:
             trace.append("gemm")
-        be.gemm(Layout.RowMajor, transA, transB, m, n, k, alpha, fa, vA.storage_offset(), lda,
-                fb, vB.storage_offset(), ldb, beta, fc, vC.storage_offset(), ldc)
+        _gemm(be, transA, transB, m, n, k, alpha, vA, lda, vB, ldb, beta, vC, ldc)
     elif (_is_contiguous_strides(vA.shape, sa) and _is_contiguous_strides(vB.shape, sb) and
           _is_contiguous_strides(vC.shape, sc)):
         if trace is not None:
             trace.append("gemmStridedBatched")
-        be.gemmStridedBatched(Layout.RowMajor, transA, transB, m, n, k, alpha,
-                              fa, vA.storage_offset(), lda, sa[-3],
-                              fb, vB.storage_offset(), ldb, sb[-3], beta,
-                              fc, vC.storage_offset(), ldc, sc[-3], batch)
+        if be is _gblas:
+            be._gemm_strided(Layout.RowMajor, transA, transB, m, n, k, alpha, be._view_operand(vA), lda, sa[-3],
+                             be._view_operand(vB), ldb, sb[-3], beta, be._view_operand(vC), ldc, sc[-3], batch)
+        else:
+            be.gemmStridedBatched(Layout.RowMajor, transA, transB, m, n, k, alpha,
+                                  _flat(vA), vA.storage_offset(), lda, sa[-3],
+                                  _flat(vB), vB.storage_offset(), ldb, sb[-3], beta,
+                                  _flat(vC), vC.storage_offset(), ldc, sc[-3], batch)
     else:
         if trace is not None:
             trace.append("gemmBatched")
         a_off = [_linear_offset(vA.shape, sa, vA.storage_offset(), p * m * k) for p in range(batch)]
         b_off = [_linear_offset(vB.shape, sb, vB.storage_offset(), p * k * n) for p in range(batch)]
         c_off = [_linear_offset(vC.shape, sc, vC.storage_offset(), p * m * n) for p in range(batch)]
-        be.gemmBatched(Layout.RowMajor, transA, transB, m, n, k, [alpha] * batch, fa, a_off, lda,
-                       fb, b_off, ldb, [beta] * batch, fc, c_off, ldc, batch)
+        be.gemmBatched(Layout.RowMajor, transA, transB, m, n, k, [alpha] * batch, _flat(vA), a_off, lda,
+                       _flat(vB), b_off, ldb, [beta] * batch, _flat(vC), c_off, ldc, batch)
     return C
 
 
