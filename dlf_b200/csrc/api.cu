@@ -22,6 +22,7 @@
 #include "channels_last.cuh"
 #include "contraction.cuh"
 #include "contraction_ts.cuh"
+#include "contraction_split.cuh"
 #include "conv_small.cuh"
 #include "conv_halo.cuh"
 #include "level3.cuh"
@@ -66,6 +67,7 @@ struct DeviceState {
     int static_smem_pair = 0;
     int static_smem_small = 0;
     int static_smem_halo = 0;
+    bool split_ready = false;   // contraction_split_kernel is set up
     int max_pair_clusters = 0;  // co-resident CTA pairs of the pair kernel (0 = not usable)
     PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
     PFN_cuTensorMapEncodeIm2col_v12000 encode_im2col = nullptr;  // null: the driver has none
@@ -164,6 +166,14 @@ cudaError_t launch_ts_kernel(const cudaLaunchConfig_t* cfg, const TsParams& tp, 
     return cudaLaunchKernelEx(cfg, contraction_ts_kernel<ES, A_DENSE_MN>, tp, tm_b, tm_d);
 }
 
+// contraction_split_kernel
+int setup_tma_kernels(DeviceState& st) {
+    for (auto k : {contraction_split_kernel<OUT_F16>, contraction_split_kernel<OUT_BF16>})
+        CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, split_smem_bytes(kSplitMaxStages)));
+    st.split_ready = true;
+    return kSuccess;
+}
+
 int ensure_device(DeviceState** out) {
     int dev = 0;
     CUDA_TRY(cudaGetDevice(&dev));
@@ -248,6 +258,10 @@ int ensure_device(DeviceState** out) {
                 std::fprintf(stderr, "dlf_b200: pair kernel static smem %d, dyn %d, max clusters %d (%s)\n",
                              st.static_smem_pair, dyn, n, cudaGetErrorString(oe));
             (void)cudaGetLastError();
+        }
+        {
+            const int rc2 = setup_tma_kernels(st);
+            if (rc2 != kSuccess) return rc2;
         }
         void* fn = nullptr;
         cudaDriverEntryPointQueryResult qres;
@@ -792,6 +806,96 @@ int launch_ts(const DeviceState& st, const Problem& q, cudaStream_t stream) {
     return kSuccess;
 }
 
+// CTAs per tile of contraction_split_kernel for a problem in its form (rows of D contiguous along q.N), or 0 when
+// the problem is not one for it: too many tiles to run at once, or an operand or output it cannot address.
+int split_ctas(const DeviceState& st, const Problem& q) {
+    if (q.es != 2 || !st.split_ready || g_force_generic.load() != 0 || g_force_bn.load() != 0 || q.d_f32 || q.cl_swap ||
+        q.a.im2col || q.rc_kw || q.a_offs != nullptr || q.b_offs != nullptr || q.d_offs != nullptr || q.alphas != nullptr ||
+        q.betas != nullptr || q.a_idx != nullptr || q.b_idx != nullptr || q.d_idx != nullptr || q.bias_rows || q.a_cl > 1)
+        return 0;
+    if (((reinterpret_cast<uintptr_t>(q.d) | reinterpret_cast<uintptr_t>(q.resid) | reinterpret_cast<uintptr_t>(q.bias)) & 15u) ||
+        q.N % 8 != 0 || q.ldd % 8 != 0 || (q.batch > 1 && q.d_batch_stride % 8 != 0) || (q.bias != nullptr && q.batch > 1))
+        return 0;
+    if (q.a_cl == 0 && !tma_ok(q.a, q.es, q.M, q.K, q.batch)) return 0;
+    if (!tma_ok(q.b, q.es, q.N, q.K, q.batch)) return 0;
+    const long long tiles = q.batch * ((q.M + kBM - 1) / kBM) * ((q.N + kSplitBN - 1) / kSplitBN);
+    if (tiles > st.num_sms) return 0;
+    const long long num_kb = (q.K + 63) / 64;
+    int s = 1;
+    // (GPCs hold whole clusters: 4 and 8 CTAs do not tile all 148 SMs)
+    while (2 * s <= kSplitMaxCtas && tiles * 2 * s <= (2 * s > 2 ? 128 : st.num_sms) && num_kb >= 8 * s) s *= 2;
+    return s;
+}
+
+int launch_split(const DeviceState& st, const Problem& q, int ctas, cudaStream_t stream) {
+    const long long num_kb = (q.K + 63) / 64;
+    const long long tiles_m = (q.M + kBM - 1) / kBM, tiles_n = (q.N + kSplitBN - 1) / kSplitBN;
+    const int stages = static_cast<int>(std::min<long long>(kSplitMaxStages, (num_kb + ctas - 1) / ctas));
+    Params p{};
+    p.M = static_cast<int>(q.M);
+    p.N = static_cast<int>(q.N);
+    p.K = static_cast<int>(q.K);
+    p.batch = static_cast<int>(q.batch);
+    p.BN = kSplitBN;
+    p.stages = stages;
+    p.fmt = q.fmt;
+    p.tiles_m = static_cast<int>(tiles_m);
+    p.tiles_n = static_cast<int>(tiles_n);
+    p.total_tiles = static_cast<int>(q.batch * tiles_m * tiles_n);
+    p.alpha = q.alpha;
+    p.beta = q.beta;
+    p.a = q.a;
+    p.b = q.b;
+    p.d = q.d;
+    p.ldd = q.ldd;
+    p.d_batch_stride = q.d_batch_stride;
+    p.bias = q.bias;
+    p.resid = q.resid;
+    p.relu = q.relu;
+    p.g = q.g;
+    p.status = st.status;
+    p.a_cl = q.a_cl;
+    p.cl_cblocks = q.cl_cblocks;
+    set_wait_policy(p, p.total_tiles);
+    CUtensorMap tm_a, tm_b;
+    int rc = q.a_cl == 1 ? encode_im2col_map(st, &tm_a, q, q.a.base, kBM) : encode_map(st, &tm_a, q.a, q.es, q.M, q.K, q.batch, kBM);
+    if (rc != kSuccess) return rc;
+    rc = encode_map(st, &tm_b, q.b, q.es, q.N, q.K, q.batch, kSplitBN);
+    if (rc != kSuccess) return rc;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(p.total_tiles * ctas), 1, 1);
+    cfg.blockDim = dim3(kSplitThreads, 1, 1);
+    cfg.dynamicSmemBytes = split_smem_bytes(stages);
+    cfg.stream = stream;
+    // programmatic dependent launch: barriers, tensor memory and tensor maps are set up while the kernel before
+    // this one still runs; nothing it may have written is touched before griddepcontrol.wait
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = static_cast<unsigned>(ctas);
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = ctas > 1 ? 2 : 1;
+    if (q.fmt == FMT_F16) CUDA_TRY(cudaLaunchKernelEx(&cfg, contraction_split_kernel<OUT_F16>, p, tm_a, tm_b, ctas));
+    else CUDA_TRY(cudaLaunchKernelEx(&cfg, contraction_split_kernel<OUT_BF16>, p, tm_a, tm_b, ctas));
+    g_launches.fetch_add(1);
+    CUDA_TRY(cudaGetLastError());
+    return kSuccess;
+}
+
+// The same product with the operands exchanged (D^T = Bu * Au^T): lanes hold the columns of D, and a row of the
+// tile runs along D's contiguous index.
+Problem exchanged(const Problem& q_in) {
+    Problem q = q_in;
+    std::swap(q.a, q.b);
+    std::swap(q.M, q.N);
+    std::swap(q.a_idx, q.b_idx);
+    std::swap(q.a_count, q.b_count);
+    return q;
+}
+
 int launch(const Problem& q_in, cudaStream_t stream, DeviceState* preset = nullptr) {
     DeviceState* st = preset;
     int rc = kSuccess;
@@ -802,6 +906,16 @@ int launch(const Problem& q_in, cudaStream_t stream, DeviceState* preset = nullp
     clear_stale_error();
     if (q_in.M > INT_MAX - 512 || q_in.N > INT_MAX - 512 || q_in.K > INT_MAX - 512 || q_in.batch > INT_MAX)
         return kInvalidDimension;
+
+    // few output tiles: one cluster per tile
+    if (q_in.es == 2 && (q_in.out_nchw == 5 || (q_in.out_nchw == 0 && q_in.a_cl == 0 && q_in.bias == nullptr && q_in.resid == nullptr))) {
+        const Problem qs = q_in.out_nchw == 5 ? q_in : exchanged(q_in);
+        const int ctas = split_ctas(*st, qs);
+        if (ctas > 0) {
+            rc = launch_split(*st, qs, ctas, stream);
+            if (rc != kNotImplemented) return rc;  // else: window corners outside the im2col map's range
+        }
+    }
 
     // A plain 16-bit product whose result can leave through TMA stores is computed transposed: with
     // the operands exchanged the lanes hold the columns j of D and the accumulator columns run along
@@ -821,10 +935,7 @@ int launch(const Problem& q_in, cudaStream_t stream, DeviceState* preset = nullp
         (q.batch == 1 || q.d_batch_stride == 0 || (q.d_batch_stride * q.es) % 16 == 0) &&
         tma_ok(q.a, q.es, q.M, q.K, q.batch) && tma_ok(q.b, q.es, q.N, q.K, q.batch) &&
         !((g_force_bn.load() >> 16) & 16384)) {
-        std::swap(q.a, q.b);
-        std::swap(q.M, q.N);
-        std::swap(q.a_idx, q.b_idx);
-        std::swap(q.a_count, q.b_count);
+        q = exchanged(q_in);
         q.out_nchw = 5;
         q.narrow_boxes = true;  // measured on the batched product above: 125-128 us with 2 KB boxes, 136 us with 4 KB ones
     }
@@ -1390,7 +1501,10 @@ int dlf_b200_gemm_ex(int dtype, int layout, int trans_a, int trans_b, size_t m, 
     DeviceState* st = nullptr;
     rc = ensure_device(&st);
     if (rc != kSuccess) return rc;
-    if (workspace != nullptr && !(g_force_generic.load() & 0x20000000)) {
+    // A product with few tiles whose operands the tensor maps take can share a tile's K range out inside one launch,
+    // over the CTAs of a cluster. A cluster has 8 at most: 16 tiles and fewer fill more SMs as slices of a launch.
+    const bool in_cluster = ((q.M + kBM - 1) / kBM) * ((q.N + 127) / 128) > 16 && split_ctas(*st, exchanged(q)) > 0;
+    if (workspace != nullptr && !(g_force_generic.load() & 0x20000000) && !in_cluster) {
         char* ws = align256(workspace);
         const size_t slack = static_cast<size_t>(ws - static_cast<char*>(workspace));
         size_t slices = splitk_slices(q, st->num_sms);
@@ -2099,9 +2213,9 @@ int dlf_b200_conv2d_fused(int dtype, size_t batches, size_t channels, size_t hei
                 if (!w_direct) {
                     const long long total = static_cast<long long>(num_kernels) * ck;
                     const unsigned blocks = static_cast<unsigned>(std::min<long long>((total + 255) / 256, 8ll * st->num_sms));
-                    cl_pack_filters_kernel<<<blocks, 256, 0, cs>>>(static_cast<const uint16_t*>(w), wp,
-                                                                  static_cast<int>(num_kernels), static_cast<int>(channels),
-                                                                  static_cast<int>(taps), static_cast<int>(ck));
+                    cl_pack_filters_kernel<<<blocks, 256, 0, cs>>>( static_cast<const uint16_t*>(w), wp,
+                                              static_cast<int>(num_kernels), static_cast<int>(channels),
+                                              static_cast<int>(taps), static_cast<int>(ck));
                     g_launches.fetch_add(1);
                     CUDA_TRY(cudaGetLastError());
                 }
@@ -2771,7 +2885,8 @@ int dlf_b200_conv2d_nhwc(int dtype, size_t batches, size_t channels, size_t heig
         // 64 output channels, where half of the lanes idle (64 -> 64 3x3 at 56x56: 146 -> 156 us;
         // 256 -> 64 1x1: 81 -> 108 us), nor for 1x1 filters (512 -> 128 at 28x28: 48 -> 50 us).
         // Bit 28 of the tile-width word: never.
-        if (num_kernels > 64 && num_kernels <= 128 && taps > 1 && !((g_force_bn.load() >> 16) & 4096)) {
+        // (Too few pixels to fill the GPU with tiles: contraction_split_kernel takes the form as it is.)
+        if (num_kernels > 64 && num_kernels <= 128 && taps > 1 && !((g_force_bn.load() >> 16) & 4096) && split_ctas(*st, q) == 0) {
             std::swap(q.a, q.b);
             q.M = static_cast<long long>(num_kernels);
             q.N = static_cast<long long>(batches) * P;

@@ -83,6 +83,12 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
     }
 }
 
+// ---------------------------------------------------------------- launches
+// Programmatic dependent launch: the next kernel of the stream may start (its CTAs wait below until this grid
+// has completed) / wait for the grids before this one.
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void wait_for_dependencies() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---------------------------------------------------------------- fences
 // Generic-proxy shared-memory writes -> visible to the async proxy (UMMA operand reads).
 __device__ __forceinline__ void fence_proxy_async_smem() {
@@ -104,6 +110,13 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
         :
         : "r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
         : "memory");
+}
+// The box's lines into L2 only: nothing arrives anywhere, and what is written to them later is what is read later.
+__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* map, int c0, int c1, int c2) {
+    asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global [%0, {%1, %2, %3}];"
+                 :
+                 : "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2)
+                 : "memory");
 }
 // Tiled-mode's sibling for convolutions: an im2col-mode load over a channels-last (N, H, W, C)
 // tensor. Starting at base pixel (w, h, n) - the top-left corner of an output's filter window - it

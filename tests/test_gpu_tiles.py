@@ -1,0 +1,123 @@
+"""GPU parity at the edges of the tiles, chunks and clusters of the kernels that products, triangular solves
+and poolings are dispatched to by size, type and alignment, against the oracle with a double accumulator."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from support import max_rel, rel_fro
+
+pytestmark = pytest.mark.gpu
+
+FP32_TOL = 1e-5
+HALF_TOL = 2e-2
+
+
+@pytest.fixture(scope="module")
+def lib():
+    import dlf_b200
+    return dlf_b200
+
+
+@pytest.fixture(autouse=True)
+def _device_status_clean(lib):
+    yield
+    lib.set_tuning(0, 0)
+    assert lib.device_status() == 0, "a device-side bounded wait timed out"
+
+
+def _round_to(a, dtype):
+    return torch.from_numpy(np.ascontiguousarray(a, dtype=np.float32)).to(dtype).float().numpy()
+
+
+def _close(got, ref, dtype):
+    if dtype == torch.float32:
+        return rel_fro(got, ref) <= FP32_TOL
+    return max_rel(got, ref) <= HALF_TOL
+
+
+def _gemm_against_oracle(dtype, m, n, k, ta, tb, alpha, beta, pad, offset, seed):
+    """One row-major call on matrices whose lines are `pad` elements longer than needed and start `offset`
+    elements into their buffers; also checks that nothing outside the m x n window changes."""
+    from dlf_b200 import gblas as gb
+    rng = np.random.default_rng(seed)
+    lda, ldb, ldc = (m if ta else k) + pad, (k if tb else n) + pad, n + pad
+    A = _round_to(rng.uniform(-1, 1, offset + (k if ta else m) * lda), dtype)
+    B = _round_to(rng.uniform(-1, 1, offset + (n if tb else k) * ldb), dtype)
+    C = _round_to(rng.normal(size=offset + m * ldc + 16), dtype)
+    TA, TB = (gb.Transpose.Trans if t else gb.Transpose.NoTrans for t in (ta, tb))
+    ref = C.copy()
+    oracle.gblas_sgemm(oracle.ROW_MAJOR, int(TA), int(TB), m, n, k, alpha, A, offset, lda, B, offset, ldb, beta, ref, offset, ldc, wide=True)
+    start = C.copy()
+    window = np.zeros(C.size, dtype=bool)
+    window[offset:offset + m * ldc].reshape(m, ldc)[:, :n] = True
+    if beta == 0:
+        start[window] = np.nan  # must not be read
+    c = torch.from_numpy(start).to(dtype).cuda()
+    gb.gemm(gb.Layout.RowMajor, TA, TB, m, n, k, alpha, torch.from_numpy(A).to(dtype).cuda(), offset, lda,
+            torch.from_numpy(B).to(dtype).cuda(), offset, ldb, beta, c, offset, ldc)
+    got = c.float().cpu().numpy()
+    assert np.array_equal(got[~window], start[~window])
+    assert _close(got[window], ref[window], dtype), (m, n, k, ta, tb, alpha, beta)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16], ids=["f16", "bf16"])
+@pytest.mark.parametrize("m,n,k", [
+    (8, 8, 8),          # one CTA, one k-block
+    (129, 72, 504),     # tile edges, seven k-blocks: not split
+    (130, 72, 520),     # nine k-blocks over two CTAs
+    (64, 2056, 1032),   # 33 tiles of 17 k-blocks over four
+    (1000, 328, 2056),  # 33 k-blocks; more than 16 tiles
+])
+def test_16_bit_products_shared_by_a_cluster(lib, dtype, m, n, k):
+    """contraction_split_kernel: row and column remainders, uneven shares of the k-blocks, beta and alpha."""
+    for ta in (False, True):
+        for tb in (False, True):
+            m8 = (m + 7) // 8 * 8 if ta else m
+            _gemm_against_oracle(dtype, m8, n, k, ta, tb, 1.0, 0.0, 0, 0, m + n + k)
+            _gemm_against_oracle(dtype, m8, n, k, ta, tb, 0.5, 0.25, 8, 8, m + n + k + 1)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16], ids=["f32", "f16"])
+@pytest.mark.parametrize("q,systems", [(1, 1), (31, 5), (32, 3), (33, 600), (64, 4), (97, 1200), (448, 2400), (1024, 6), (1025, 5)])
+def test_triangular_solves_at_the_edges_of_their_blocks(lib, dtype, q, systems):
+    """l3_trsm_kernel: partly filled blocks of 32 unknowns, each number of systems per CTA, both contiguous
+    directions, both substitution orders, the largest order of one launch and one more."""
+    from dlf_b200 import gblas as gb
+    rng = np.random.default_rng(q + systems)
+    for side in (gb.Side.Left, gb.Side.Right):
+        m, n = (q, systems) if side == gb.Side.Left else (systems, q)
+        for tri in (gb.Triangle.Upper, gb.Triangle.Lower):
+            for ta in (gb.Transpose.NoTrans, gb.Transpose.Trans):
+                lda, ldb = q + 1, n + 3
+                A = (0.5 / np.sqrt(q)) * rng.uniform(-1, 1, (q, lda)).astype(np.float32)
+                A[np.arange(q), np.arange(q)] = rng.uniform(1.0, 2.0, q).astype(np.float32)
+                A = _round_to(A, dtype)
+                ii, jj = np.indices(A.shape)
+                keep = (jj < q) & ((ii <= jj) if tri == gb.Triangle.Upper else (ii >= jj))
+                B = _round_to(rng.uniform(-1, 1, m * ldb), dtype)
+                ref = B.copy()
+                oracle.trsm(int(side), int(tri), int(ta), int(gb.Diagonal.NonUnit), m, n, 0.5,
+                            np.where(keep, A, 0.0).astype(np.float32).ravel(), lda, ref, ldb, wide=True)
+                got = torch.from_numpy(B.copy()).to(dtype).cuda()
+                gb.trsm(gb.Layout.RowMajor, side, tri, ta, gb.Diagonal.NonUnit, m, n, 0.5,
+                        torch.from_numpy(np.where(keep, A, np.nan).astype(np.float32).ravel()).to(dtype).cuda(), 0, lda, got, 0, ldb)
+                g = got.float().cpu().numpy()
+                if dtype == torch.float32:
+                    assert rel_fro(g, ref) <= FP32_TOL, (side, tri, ta)
+                else:
+                    assert max_rel(g, ref) <= 5e-2, (side, tri, ta)
+
+
+def test_triangular_solve_with_a_zero_and_an_infinite_pivot(lib):
+    """What IEEE division gives: x / 0 = inf, 0 / 0 = NaN, x / inf = 0, and nothing spreads backwards."""
+    from dlf_b200 import gblas as gb
+    n = 40
+    T = torch.eye(n, device="cuda")
+    T[5, 5], T[7, 7], T[36, 36] = 0.0, float("inf"), 2.0
+    B = torch.ones(n, 3, device="cuda")
+    B[5, 1] = 0.0
+    gb.trsm(gb.Layout.RowMajor, gb.Side.Left, gb.Triangle.Lower, gb.Transpose.NoTrans, gb.Diagonal.NonUnit, n, 3, 1.0,
+            T.view(-1), 0, n, B.view(-1), 0, 3)
+    got = B.cpu()
+    assert torch.isinf(got[5, 0]) and torch.isnan(got[5, 1]) and bool((got[:5] == 1.0).all())
