@@ -22,6 +22,7 @@
 #include "channels_last.cuh"
 #include "contraction.cuh"
 #include "contraction_ts.cuh"
+#include "contraction_f32.cuh"
 #include "contraction_split.cuh"
 #include "conv_small.cuh"
 #include "conv_halo.cuh"
@@ -68,6 +69,8 @@ struct DeviceState {
     int static_smem_small = 0;
     int static_smem_halo = 0;
     bool split_ready = false;   // contraction_split_kernel is set up
+    int static_smem_f32 = -1;   // contraction_f32_kernel; -1: not set up on this path
+    int max_f32_clusters[9] = {0};  // co-resident clusters of [size] CTAs that share a tile's k-blocks
     int max_pair_clusters = 0;  // co-resident CTA pairs of the pair kernel (0 = not usable)
     PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
     PFN_cuTensorMapEncodeIm2col_v12000 encode_im2col = nullptr;  // null: the driver has none
@@ -166,8 +169,35 @@ cudaError_t launch_ts_kernel(const cudaLaunchConfig_t* cfg, const TsParams& tp, 
     return cudaLaunchKernelEx(cfg, contraction_ts_kernel<ES, A_DENSE_MN>, tp, tm_b, tm_d);
 }
 
+// contraction_f32_kernel (shared memory of every instantiation, clusters that fit on the GPU) and
 // contraction_split_kernel
 int setup_tma_kernels(DeviceState& st) {
+    cudaFuncAttributes fa;
+    int worst = 0;
+    for (auto k : {contraction_f32_kernel<1>, contraction_f32_kernel<2>, contraction_f32_kernel<3>}) {
+        CUDA_TRY(cudaFuncGetAttributes(&fa, k));
+        worst = std::max(worst, static_cast<int>(fa.sharedSizeBytes));
+    }
+    for (auto k : {contraction_f32_kernel<1>, contraction_f32_kernel<2>, contraction_f32_kernel<3>})
+        CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemPerBlockOptin - worst));
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(kF32Threads, 1, 1);
+    cfg.dynamicSmemBytes = static_cast<size_t>(kSmemPerBlockOptin - worst);
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    st.max_f32_clusters[1] = st.num_sms;
+    for (int size = 2; size <= 8; ++size) {
+        attr.val.clusterDim.x = static_cast<unsigned>(size);
+        cfg.gridDim = dim3(static_cast<unsigned>(size * st.num_sms), 1, 1);
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, contraction_f32_kernel<3>, &cfg) == cudaSuccess) st.max_f32_clusters[size] = n;
+    }
+    (void)cudaGetLastError();
+    st.static_smem_f32 = worst;
     for (auto k : {contraction_split_kernel<OUT_F16>, contraction_split_kernel<OUT_BF16>})
         CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, split_smem_bytes(kSplitMaxStages)));
     st.split_ready = true;
@@ -806,6 +836,122 @@ int launch_ts(const DeviceState& st, const Problem& q, cudaStream_t stream) {
     return kSuccess;
 }
 
+// Whether a problem can go to contraction_f32_kernel: both operands through tensor maps, one alpha and beta, plain
+// output. Any tuning bit of the operand paths keeps the general fp32 kernel, which those bits belong to.
+bool f32_tma_ok(const DeviceState& st, const Problem& q) {
+    return q.es == 4 && st.static_smem_f32 >= 0 && g_force_generic.load() == 0 && q.a_cl == 0 && (q.out_nchw == 0 || q.out_nchw == 1) &&
+           !q.a.im2col && !q.rc_kw && q.a_offs == nullptr && q.b_offs == nullptr && q.d_offs == nullptr &&
+           q.alphas == nullptr && q.betas == nullptr && q.a_idx == nullptr && q.b_idx == nullptr && q.d_idx == nullptr &&
+           (q.bias == nullptr || (!q.bias_rows && q.bias_stride == 0 && q.alpha == 1.0f)) && tma_ok(q.a, q.es, q.M, q.K, q.batch) && tma_ok(q.b, q.es, q.N, q.K, q.batch);
+}
+
+// tensor map of the MN-major A operand of contraction_f32_kernel: boxes of 128 rows x 32 k, not swizzled (a lane
+// of a splitter warp reads one row)
+int encode_f32_rows_map(const DeviceState& st, CUtensorMap* map, const Problem& q) {
+    const GenOperand& op = q.a;
+    const bool batched = q.batch > 1 && op.batch_stride != 0;
+    const cuuint64_t ld = op.ld > 0 && (op.ld * 4) % 16 == 0 ? static_cast<cuuint64_t>(op.ld) * 4 : 16;
+    cuuint64_t dims[3] = {static_cast<cuuint64_t>(q.M), static_cast<cuuint64_t>(q.K), static_cast<cuuint64_t>(batched ? q.batch : 1)};
+    cuuint64_t strides[2] = {ld, batched ? static_cast<cuuint64_t>(op.batch_stride) * 4 : ld * dims[1]};
+    if (strides[1] >= (1ull << 40)) strides[1] = ld;
+    cuuint32_t box[3] = {kBM, 32, 1}, estr[3] = {1, 1, 1};
+    const CUresult r = st.encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<char*>(op.base), dims, strides, box, estr,
+                                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? kSuccess : kUnexpectedError;
+}
+
+int launch_f32(const DeviceState& st, const Problem& q, cudaStream_t stream) {
+    const long long num_kb = (q.K + 31) / 32;
+    // The width with the least (waves of tiles) x (clocks of a tile); clocks per k-block measured at 4096^3
+    // (960, 650 and 590 us), the write of a tile about 30 clocks a column.
+    static const double kb_clk[4] = {0.0, 1020.0, 1380.0, 1750.0};
+    const int forced = g_force_bn.load() & 0xffff;  // 64, 128, 192
+    const long long tiles_m = (q.M + kBM - 1) / kBM;
+    double best_cost = 0;
+    int nb = 0, split = 1;
+    for (int w = 1; w <= 3; ++w) {
+        if (forced % 64 == 0 && forced >= 64 && forced <= 192 && forced != 64 * w) continue;
+        const long long tiles = q.batch * tiles_m * ((q.N + 64 * w - 1) / (64 * w));
+        const double write_clk = 30.0 * 64 * w;
+        // few tiles: a cluster per tile, its k-blocks shared out, at least four each (the cluster's launch and
+        // the exchange of the partial tiles: 5 us, 9000 clocks; 1024^3 20.7 us without, 23.5 us with two CTAs of 128 columns)
+        for (int sp = 1; sp <= 8; ++sp) {
+            if (sp > 1 && (tiles > st.max_f32_clusters[sp] || num_kb < 4 * sp)) continue;
+            const double waves = static_cast<double>((tiles + st.num_sms - 1) / st.num_sms);
+            const double cost = waves * (static_cast<double>((num_kb + sp - 1) / sp) * kb_clk[w] + write_clk) + (sp > 1 ? 9000.0 : 0.0);
+            if (nb == 0 || cost < best_cost) {
+                nb = w;
+                best_cost = cost;
+                split = sp;
+            }
+        }
+    }
+    if (nb == 0) return kUnexpectedError;
+    const int bn = 64 * nb;
+    const long long tiles_n = (q.N + bn - 1) / bn;
+    const long long total = q.batch * tiles_m * tiles_n;
+    if (total >= INT_MAX) return kInvalidDimension;
+    const int stage = f32_stage_bytes(nb);
+    const int stages = std::min(kF32MaxStages, (kSmemPerBlockOptin - st.static_smem_f32 - 1024) / stage);
+    if (stages < 2) return kUnexpectedError;
+
+    Params p{};
+    p.M = static_cast<int>(q.M);
+    p.N = static_cast<int>(q.N);
+    p.K = static_cast<int>(q.K);
+    p.batch = static_cast<int>(q.batch);
+    p.BN = bn;
+    p.stages = stages;
+    p.fmt = q.fmt;
+    p.tiles_m = static_cast<int>(tiles_m);
+    p.tiles_n = static_cast<int>(tiles_n);
+    p.total_tiles = static_cast<int>(total);
+    p.alpha = q.alpha;
+    p.beta = q.beta;
+    p.a = q.a;
+    p.b = q.b;
+    p.d = q.d;
+    p.ldd = q.ldd;
+    p.d_batch_stride = q.d_batch_stride;
+    p.bias = q.bias;
+    p.resid = q.resid;
+    p.relu = q.relu;
+    p.out_nchw = q.out_nchw;
+    p.g = q.g;
+    p.status = st.status;
+    set_wait_policy(p, total);
+    CUtensorMap tm_a, tm_b;
+    int rc = q.a.k_major ? encode_map(st, &tm_a, q.a, 4, q.M, q.K, q.batch, kBM) : encode_f32_rows_map(st, &tm_a, q);
+    if (rc != kSuccess) return rc;
+    rc = encode_map(st, &tm_b, q.b, 4, q.N, q.K, q.batch, bn);
+    if (rc != kSuccess) return rc;
+
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(split > 1 ? total * split : std::min<long long>(total, st.num_sms)), 1, 1);
+    cfg.blockDim = dim3(kF32Threads, 1, 1);
+    cfg.dynamicSmemBytes = static_cast<size_t>(stages) * stage + 1024;
+    cfg.stream = stream;
+    // (programmatic dependent launch: see launch_split)
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = static_cast<unsigned>(split);
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = split > 1 ? 2 : 1;
+    if (std::getenv("DLF_B200_DEBUG"))
+        std::fprintf(stderr, "dlf_b200: f32 launch bn=%d split=%d tiles=%lld stages=%d clusters 2:%d 3:%d 4:%d 8:%d\n", bn, split, total,
+                     stages, st.max_f32_clusters[2], st.max_f32_clusters[3], st.max_f32_clusters[4], st.max_f32_clusters[8]);
+    const auto kernel = nb == 1 ? contraction_f32_kernel<1> : nb == 2 ? contraction_f32_kernel<2> : contraction_f32_kernel<3>;
+    CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, p, tm_a, tm_b, split));
+    g_launches.fetch_add(1);
+    CUDA_TRY(cudaGetLastError());
+    return kSuccess;
+}
+
 // CTAs per tile of contraction_split_kernel for a problem in its form (rows of D contiguous along q.N), or 0 when
 // the problem is not one for it: too many tiles to run at once, or an operand or output it cannot address.
 int split_ctas(const DeviceState& st, const Problem& q) {
@@ -944,7 +1090,8 @@ int launch(const Problem& q_in, cudaStream_t stream, DeviceState* preset = nullp
                          ((q.a_cl != 0 && !q.cl_swap) || tma_ok(q.a, q.es, q.M, q.K, q.batch)) &&
                          ((q.a_cl != 0 && q.cl_swap) || tma_ok(q.b, q.es, q.N, q.K, q.batch));
     if (q.a_cl != 0 && !use_tma) return kNotImplemented;
-    // A through tensor memory: every convolution and every fp32 product (see contraction_ts.cuh)
+    if (f32_tma_ok(*st, q)) return launch_f32(*st, q, stream);
+    // A through tensor memory: every convolution and every other fp32 product (see contraction_ts.cuh)
     const int force_path = g_force_generic.load() & 0xff;
     if (force_path != 2 && !q.no_ts && !use_tma && (q.a.im2col || q.es == 4 || force_path == 3)) {
         rc = launch_ts(*st, q, stream);
@@ -1503,7 +1650,7 @@ int dlf_b200_gemm_ex(int dtype, int layout, int trans_a, int trans_b, size_t m, 
     if (rc != kSuccess) return rc;
     // A product with few tiles whose operands the tensor maps take can share a tile's K range out inside one launch,
     // over the CTAs of a cluster. A cluster has 8 at most: 16 tiles and fewer fill more SMs as slices of a launch.
-    const bool in_cluster = ((q.M + kBM - 1) / kBM) * ((q.N + 127) / 128) > 16 && split_ctas(*st, exchanged(q)) > 0;
+    const bool in_cluster = ((q.M + kBM - 1) / kBM) * ((q.N + 127) / 128) > 16 && (split_ctas(*st, exchanged(q)) > 0 || f32_tma_ok(*st, q));
     if (workspace != nullptr && !(g_force_generic.load() & 0x20000000) && !in_cluster) {
         char* ws = align256(workspace);
         const size_t slack = static_cast<size_t>(ws - static_cast<char*>(workspace));
@@ -1749,6 +1896,11 @@ size_t dlf_b200_conv2d_workspace_bytes(int dtype, size_t batches, size_t channel
     const size_t row = group * ((ng + 255) / 256 * 256 + 256) * 128 * dup *
                        ((cg * kernel_h * (kernel_w + 8) + bk - 1) / bk + 8);
     size_t need = (plain > row ? plain : row) + 256;
+    // fp32 1x1 filters: the kept pixels with their channels contiguous
+    if (es == 4 && group == 1 && kernel_h == 1 && kernel_w == 1) {
+        const size_t cl = batches * height * width * channels * 4 + 512;
+        if (cl > need) need = cl;
+    }
     // channels-last route (16-bit, one group): channels-last copy of the activations plus the
     // filter bank in (tap, channel) order
     if (es == 2 && group == 1) {
@@ -1818,7 +1970,8 @@ int dlf_b200_conv2d_fused(int dtype, size_t batches, size_t channels, size_t hei
     // exactly the reference's convWithIm2Col shortcut (gpgpu/src/gdnn.cpp:1512-1559: weights
     // shared with stride 0). With TMA-compatible strides it takes the TMA-fed kernel.
     if (kernel_h == 1 && kernel_w == 1 && stride_h == 1 && stride_w == 1 && pad_top == 0 &&
-        pad_left == 0 && output_h == height && output_w == width && group == 1 && q.es == 2 &&
+        pad_left == 0 && output_h == height && output_w == width && group == 1 &&
+        (q.es == 2 || (g_force_generic.load() == 0 && g_force_bn.load() == 0 && P <= INT_MAX / 2)) &&
         (P * q.es) % 16 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 &&
         (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && (channels * q.es) % 16 == 0 &&
         !(g_force_generic.load() & 0xff)) {
@@ -1848,7 +2001,7 @@ int dlf_b200_conv2d_fused(int dtype, size_t batches, size_t channels, size_t hei
         // cheaper ones (64 -> 64 at 56x56: 69 -> 63 us; 256 -> 64: 93 -> 92 us). Bit 19 of the
         // tile-width word: never swap.
         const uintptr_t ya = reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(residual);
-        if (P % 8 == 0 && P >= 32 && ya % 16 == 0 && num_kernels >= 64 && !((g_force_bn.load() >> 16) & 8)) {
+        if (q.es == 2 && P % 8 == 0 && P >= 32 && ya % 16 == 0 && num_kernels >= 64 && !((g_force_bn.load() >> 16) & 8)) {
             std::swap(q.a, q.b);
             q.M = static_cast<long long>(num_kernels);
             q.N = P;
@@ -1859,6 +2012,50 @@ int dlf_b200_conv2d_fused(int dtype, size_t batches, size_t channels, size_t hei
             q.g.out_img_stride = static_cast<long long>(num_kernels) * P;
         }
         return launch(q, static_cast<cudaStream_t>(stream));
+    }
+
+    // Other 1x1 filters without padding on fp32 data (a stride, or planes that are no 16-byte multiple): the kept
+    // pixels are copied with their channels contiguous, after which the layer is one product over all images,
+    // written to NCHW by lanes that hold pixels. (ResNet-50 at batch 8 has eleven such layers: 30 us each by the
+    // gathering kernel; the whole forward 1416 -> 1274 us.)
+    if (q.es == 4 && group == 1 && kernel_h == 1 && kernel_w == 1 && pad_top == 0 && pad_left == 0 && channels % 4 == 0 &&
+        (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && (output_h - 1) * stride_h < height && (output_w - 1) * stride_w < width &&
+        workspace != nullptr && g_force_generic.load() == 0 && g_force_bn.load() == 0 && batches < 65536 &&
+        static_cast<long long>(batches) * P < INT_MAX - 512 && (channels + 31) / 32 < 65536 && channels < INT_MAX - 512 &&
+        num_kernels < INT_MAX - 512 && static_cast<long long>(height) * width < INT_MAX) {
+        char* xp = align256(workspace);
+        const size_t need = static_cast<size_t>(xp - static_cast<char*>(workspace)) + batches * static_cast<size_t>(P) * channels * 4;
+        DeviceState* st = nullptr;
+        int rc = ensure_device(&st);
+        if (rc != kSuccess) return rc;
+        if (workspace_bytes >= need && st->static_smem_f32 >= 0) {
+            clear_stale_error();
+            const dim3 grid(static_cast<unsigned>((P + 31) / 32), static_cast<unsigned>((channels + 31) / 32), static_cast<unsigned>(batches));
+            f32_pack_pixels_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+                static_cast<const float*>(x), reinterpret_cast<float*>(xp), static_cast<int>(channels),
+                static_cast<long long>(height) * width, static_cast<int>(width), static_cast<int>(P), static_cast<int>(output_w),
+                static_cast<int>(stride_h), static_cast<int>(stride_w));
+            g_launches.fetch_add(1);
+            CUDA_TRY(cudaGetLastError());
+            q.M = static_cast<long long>(batches) * P;
+            q.N = static_cast<long long>(num_kernels);
+            q.K = static_cast<long long>(channels);
+            q.a.base = xp;
+            q.a.k_major = 1;
+            q.a.ld = static_cast<long long>(channels);
+            q.b.base = static_cast<const char*>(w);
+            q.b.k_major = 1;
+            q.b.ld = static_cast<long long>(channels);
+            q.d = static_cast<char*>(y);
+            q.ldd = P;
+            q.bias = static_cast<const char*>(bias);
+            q.out_nchw = 1;
+            q.g.P = static_cast<int>(P);
+            q.g.out_img_stride = static_cast<long long>(num_kernels) * P;
+            q.pack_ws = nullptr;
+            q.pack_ws_bytes = 0;
+            return launch(q, static_cast<cudaStream_t>(stream), st);
+        }
     }
 
     q.M = static_cast<long long>(batches) * P;  // global output pixel index

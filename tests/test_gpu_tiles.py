@@ -61,6 +61,22 @@ def _gemm_against_oracle(dtype, m, n, k, ta, tb, alpha, beta, pad, offset, seed)
     assert _close(got[window], ref[window], dtype), (m, n, k, ta, tb, alpha, beta)
 
 
+@pytest.mark.parametrize("width", [0, 64, 128, 192])
+@pytest.mark.parametrize("m,n,k", [
+    (4, 8, 4),          # one partly filled tile, less than a k-block
+    (129, 132, 260),    # a row and four columns into the next tile, a ninth k-block: a second chunk of one
+    (196, 260, 256),    # exactly one chunk
+    (68, 196, 1028),    # clusters: the last CTA's share is longer
+])
+def test_fp32_products_through_tensor_maps(lib, width, m, n, k):
+    """contraction_f32_kernel at every tile width, all transposes, with and without beta."""
+    lib.set_tuning(width, 0)
+    for ta in (False, True):
+        for tb in (False, True):
+            _gemm_against_oracle(torch.float32, m, 4 * ((n + 3) // 4), k, ta, tb, 1.0, 0.0, 0, 0, m + n + k)
+            _gemm_against_oracle(torch.float32, 4 * ((m + 3) // 4), 4 * ((n + 3) // 4), k, ta, tb, 0.5, 0.25, 4, 4, m + n + k + 1)
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16], ids=["f16", "bf16"])
 @pytest.mark.parametrize("m,n,k", [
     (8, 8, 8),          # one CTA, one k-block
