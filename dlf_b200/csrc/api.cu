@@ -1428,6 +1428,71 @@ int setup_gemm(Problem& q, int dtype, int layout, int ta, int tb, size_t m, size
 
 }  // namespace
 
+// Operands that break the tensor maps' alignment rules cost a product the TMA-fed kernels: the loader warps that
+// stand in move 2 or 4 bytes an instruction. With scratch from the caller such operands are first copied with
+// their lines on 16-byte boundaries (pad_lines_kernel).
+namespace {
+
+struct PadPlan {
+    bool a = false, b = false;
+    size_t a_bytes = 0, b_bytes = 0;
+    size_t bytes() const { return a_bytes + b_bytes; }
+};
+
+size_t padded_line(long long elements, int es) { return static_cast<size_t>((elements * es + 15) / 16 * 16); }
+
+PadPlan pad_plan(const Problem& q) {
+    PadPlan plan;
+    const bool a = !tma_ok(q.a, q.es, q.M, q.K, 1), b = !tma_ok(q.b, q.es, q.N, q.K, 1);
+    if ((!a && !b) || g_force_generic.load() != 0 || q.M > INT_MAX || q.N > INT_MAX || q.K > INT_MAX) return plan;
+    // k-blocks one CTA walks: below the line the copy's launch costs more than the loader warps do
+    // (bf16 1111 x 1537 x 777, 13 blocks: 62 us by the loader warps, 6 + 11 us with the copy; fp32 60 x 72 x 50,
+    // two blocks: 11.5 us by the loader warps, and the copy's launch alone takes 3)
+    const long long tiles = ((q.M + kBM - 1) / kBM) * ((q.N + 127) / 128);
+    const long long walk = (tiles + 147) / 148 * ((q.K * q.es + 127) / 128);
+    if (walk < 4) return plan;
+    plan.a = a;
+    plan.b = b;
+    const auto too_large = [&](const GenOperand& op, long long rows) {  // the copy counts 16-byte chunks in 32 bits
+        return static_cast<double>(padded_line(op.k_major ? q.K : rows, q.es) / 16) * static_cast<double>(op.k_major ? rows : q.K) >= 2147483648.0;
+    };
+    if (too_large(q.a, q.M) || too_large(q.b, q.N)) return PadPlan();
+    if (a) plan.a_bytes = padded_line(q.a.k_major ? q.K : q.M, q.es) * static_cast<size_t>(q.a.k_major ? q.M : q.K);
+    if (b) plan.b_bytes = padded_line(q.b.k_major ? q.K : q.N, q.es) * static_cast<size_t>(q.b.k_major ? q.N : q.K);
+    return plan;
+}
+
+// copies the operands the plan names into `ws` and points the problem at the copies
+int pad_operands(Problem& q, const PadPlan& plan, char* ws, cudaStream_t stream) {
+    PadLines p{};
+    int n = 0;
+    long long most = 0;
+    auto add = [&](GenOperand& op, long long rows, size_t bytes) {
+        p.src[n] = op.base;
+        p.dst[n] = ws;
+        p.src_pitch[n] = op.ld * q.es;
+        p.lines[n] = op.k_major ? rows : q.K;
+        p.length[n] = static_cast<int>(op.k_major ? q.K : rows);
+        p.dst_pitch[n] = static_cast<long long>(padded_line(p.length[n], q.es));
+        most = std::max(most, p.lines[n] * p.dst_pitch[n] / 16);
+        op.base = ws;
+        op.ld = p.dst_pitch[n] / q.es;
+        ws += bytes;
+        ++n;
+    };
+    if (plan.a) add(q.a, q.M, plan.a_bytes);
+    if (plan.b) add(q.b, q.N, plan.b_bytes);
+    clear_stale_error();
+    const dim3 grid(static_cast<unsigned>(std::min<long long>((most + 255) / 256, 148 * 8)), static_cast<unsigned>(n));
+    if (q.es == 2) pad_lines_kernel<2><<<grid, 256, 0, stream>>>(p);
+    else pad_lines_kernel<4><<<grid, 256, 0, stream>>>(p);
+    g_launches.fetch_add(1);
+    CUDA_TRY(cudaGetLastError());
+    return kSuccess;
+}
+
+}  // namespace
+
 // ---------------------------------------------------------------------------------------------
 // K-split GEMM. A product with few output tiles and a long K leaves most SMs idle (the fully
 // connected layer 256 x 1000 x 2048: 16 tiles on 148 SMs). With scratch from the caller the K range
@@ -1632,6 +1697,16 @@ size_t dlf_b200_gemm_workspace_bytes(int dtype, size_t m, size_t n, size_t k) {
     return 8 * m * n * sizeof(float) + 256;
 }
 
+size_t dlf_b200_gemm_scratch_bytes(int dtype, int layout, int trans_a, int trans_b, size_t m, size_t n, size_t k,
+                                   const void* a, size_t a_ld, const void* b, size_t b_ld) {
+    Problem q;
+    char none = 0;
+    if (setup_gemm(q, dtype, layout, trans_a, trans_b, m, n, k, a, a_ld, b, b_ld, &none, layout == DLF_B200_ROW_MAJOR ? n : m) != kSuccess)
+        return 0;
+    const size_t pad = pad_plan(q).bytes();
+    return dlf_b200_gemm_workspace_bytes(dtype, m, n, k) + (pad ? pad + 512 : 0);
+}
+
 int dlf_b200_gemm_ex(int dtype, int layout, int trans_a, int trans_b, size_t m, size_t n, size_t k,
                      const void* alpha, const void* a, size_t a_ld, const void* b, size_t b_ld,
                      const void* beta, void* c, size_t c_ld, void* workspace, size_t workspace_bytes,
@@ -1648,6 +1723,17 @@ int dlf_b200_gemm_ex(int dtype, int layout, int trans_a, int trans_b, size_t m, 
     DeviceState* st = nullptr;
     rc = ensure_device(&st);
     if (rc != kSuccess) return rc;
+    if (workspace != nullptr) {
+        const PadPlan plan = pad_plan(q);
+        char* ws = align256(workspace);
+        const size_t need = static_cast<size_t>(ws - static_cast<char*>(workspace)) + plan.bytes();
+        if (plan.bytes() > 0 && workspace_bytes >= need) {
+            rc = pad_operands(q, plan, ws, s);
+            if (rc != kSuccess) return rc;
+            workspace = ws + plan.bytes();
+            workspace_bytes -= need;
+        }
+    }
     // A product with few tiles whose operands the tensor maps take can share a tile's K range out inside one launch,
     // over the CTAs of a cluster. A cluster has 8 at most: 16 tiles and fewer fill more SMs as slices of a launch.
     const bool in_cluster = ((q.M + kBM - 1) / kBM) * ((q.N + 127) / 128) > 16 && (split_ctas(*st, exchanged(q)) > 0 || f32_tma_ok(*st, q));

@@ -160,10 +160,11 @@ def _caller_scratch(device, nbytes):
     return buf
 
 
-def _gemm_workspace(device, queue, handle, nbytes):
+def _gemm_workspace(device, queue, handle, nbytes, at_least):
     """One scratch buffer per (device, stream), grown on demand; calls on a stream are ordered, so
-    they can share it. `handle` is the stream's handle, `queue` the stream (None = the current one)."""
-    own = _caller_scratch(device, nbytes)
+    they can share it. `handle` is the stream's handle, `queue` the stream (None = the current one).
+    A buffer of the caller's (`scratch`) need only hold `at_least`: the call makes do with it."""
+    own = _caller_scratch(device, at_least)
     if own is not None:
         return own
     key = (device.index, handle)
@@ -263,10 +264,15 @@ def _gemm(layout, a_transpose, b_transpose, m, n, k, alpha, a, a_ld, b, b_ld, be
         raise BLASError(StatusCode.kInvalidMatrixA)
     L = lib()
     handle = _raw_stream(queue)
-    # scratch for a K-split of products with few output tiles (the reference's Xgemm takes its
-    # temporaries from the context's pool, routines/level3/xgemm.cpp:107-223); 0 bytes = not useful
-    need = L.dlf_b200_gemm_workspace_bytes(int(prec), m, n, k)
-    ws = _gemm_workspace(c.device, queue, handle, need) if need else None
+    # scratch for a K-split of products with few output tiles and for aligned copies of operands (the
+    # reference's Xgemm takes its temporaries from the context's pool, routines/level3/xgemm.cpp:107-223);
+    # 0 bytes = not useful
+    need = L.dlf_b200_gemm_scratch_bytes(int(prec), int(layout), int(a_transpose), int(b_transpose), m, n, k,
+                                         a.address, a_ld, b.address, b_ld)
+    ws = None
+    if need:
+        least = L.dlf_b200_gemm_workspace_bytes(int(prec), m, n, k) if getattr(_SCRATCH, "buffer", None) is not None else 0
+        ws = _gemm_workspace(c.device, queue, handle, need, least)
     if event is not None:
         s = queue if queue is not None else torch.cuda.current_stream()
         event.start.record(s)

@@ -64,6 +64,11 @@ int dlf_b200_gemm_ex(int dtype, int layout, int trans_a, int trans_b, size_t m, 
                      const void* beta, void* c, size_t c_ld, void* workspace, size_t workspace_bytes,
                      void* stream);
 size_t dlf_b200_gemm_workspace_bytes(int dtype, size_t m, size_t n, size_t k);
+/* The same for one particular call: what dlf_b200_gemm_ex can use when A or B starts or continues off
+ * 16-byte boundaries is more, because it then first copies that operand with aligned lines (the
+ * products run without the extra scratch too, through slower loads). Never less than the above. */
+size_t dlf_b200_gemm_scratch_bytes(int dtype, int layout, int trans_a, int trans_b, size_t m, size_t n, size_t k,
+                                   const void* a, size_t a_ld, const void* b, size_t b_ld);
 
 /* Same product for batch_count matrices spaced by fixed strides; a stride of 0 shares one
  * operand between all batches. Replaces gpgpu::blas::gemmStridedBatched<T>

@@ -94,6 +94,30 @@ def test_16_bit_products_shared_by_a_cluster(lib, dtype, m, n, k):
             _gemm_against_oracle(dtype, m8, n, k, ta, tb, 0.5, 0.25, 8, 8, m + n + k + 1)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16], ids=["f32", "f16", "bf16"])
+@pytest.mark.parametrize("m,n,k", [(129, 131, 515), (7, 1031, 1027), (333, 111, 2049)])
+def test_products_of_operands_off_16_byte_boundaries(lib, dtype, m, n, k):
+    """Odd leading dimensions and offsets: the operands are copied with aligned lines first
+    (pad_lines_kernel); one operand aligned and the other not; offsets of every residue."""
+    for ta in (False, True):
+        for tb in (False, True):
+            for pad, offset in ((0, 0), (1, 1), (2, 3), (3, 6)):
+                _gemm_against_oracle(dtype, m, n, k, ta, tb, 1.0, 0.0, pad, offset, m + n + k)
+    _gemm_against_oracle(dtype, m + 8 - m % 8, n, k, True, False, 0.5, 0.25, 0, 0, m + n + k)
+
+
+def test_a_products_scratch_covers_its_aligned_copies(lib):
+    """dlf_b200_gemm_scratch_bytes is dlf_b200_gemm_workspace_bytes plus the copies a call needs; without
+    scratch the same call runs in one launch."""
+    L = lib.lib()
+    a = torch.zeros(200 * 515, dtype=torch.float16, device="cuda")
+    common = (16, 101, 111, 111, 150, 160, 512)
+    base = L.dlf_b200_gemm_workspace_bytes(16, 150, 160, 512)
+    assert L.dlf_b200_gemm_scratch_bytes(*common, a.data_ptr(), 512, a.data_ptr(), 160) == base
+    more = L.dlf_b200_gemm_scratch_bytes(*common, a.data_ptr() + 2, 512, a.data_ptr(), 160)
+    assert more >= base + 150 * 512 * 2
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16], ids=["f32", "f16"])
 @pytest.mark.parametrize("q,systems", [(1, 1), (31, 5), (32, 3), (33, 600), (64, 4), (97, 1200), (448, 2400), (1024, 6), (1025, 5)])
 def test_triangular_solves_at_the_edges_of_their_blocks(lib, dtype, q, systems):
