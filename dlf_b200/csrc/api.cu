@@ -836,6 +836,22 @@ int launch_ts(const DeviceState& st, const Problem& q, cudaStream_t stream) {
     return kSuccess;
 }
 
+// launch of a programmatic dependent of the kernel before it in the stream
+template <typename... Formal, typename... Actual>
+cudaError_t launch_dependent(void (*kernel)(Formal...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, Actual... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.blockDim = dim3(block, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Formal>(args)...);
+}
+
 // Whether a problem can go to contraction_f32_kernel: both operands through tensor maps, one alpha and beta, plain
 // output. Any tuning bit of the operand paths keeps the general fp32 kernel, which those bits belong to.
 bool f32_tma_ok(const DeviceState& st, const Problem& q) {
@@ -1280,12 +1296,25 @@ int launch(const Problem& q_in, cudaStream_t stream, DeviceState* preset = nullp
     }
 
     const unsigned grid = static_cast<unsigned>(total < st->num_sms ? total : st->num_sms);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.dynamicSmemBytes = dyn_smem;
+    cfg.stream = stream;
+    // Programmatic dependent launch (see launch_split) for convolutions, which follow one another in a network
+    // (forward of 256 images 4092 -> 4063 us), and for products of at most two waves of tiles; longer products gain
+    // nothing by it (4096^3 125.1 / 125.9 us, 1024 x (512 x 512 x 64) 131.8 / 133.2 us without / with).
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = q_in.out_nchw != 0 || q_in.a_cl != 0 || total <= 2ll * st->num_sms ? 1 : 0;
     if (use_tma) {
 #define DLF_TMA_LAUNCH(ESETS)                                                                                      \
+        cfg.blockDim = dim3(tma_threads(ESETS), 1, 1);                                                             \
         if (p.r_tma)                                                                                               \
-            contraction_kernel<2, true, false, ESETS, true><<<grid, tma_threads(ESETS), dyn_smem, stream>>>(p, tm_a, tm_b, tm_d, tm_r); \
+            CUDA_TRY(cudaLaunchKernelEx(&cfg, contraction_kernel<2, true, false, ESETS, true>, p, tm_a, tm_b, tm_d, tm_r)); \
         else                                                                                                       \
-            contraction_kernel<2, true, false, ESETS, false><<<grid, tma_threads(ESETS), dyn_smem, stream>>>(p, tm_a, tm_b, tm_d, tm_r)
+            CUDA_TRY(cudaLaunchKernelEx(&cfg, contraction_kernel<2, true, false, ESETS, false>, p, tm_a, tm_b, tm_d, tm_r))
         if (four_sets) {
             DLF_TMA_LAUNCH(4);
         } else if (three_sets) {
@@ -2243,9 +2272,9 @@ int dlf_b200_conv2d_fused(int dtype, size_t batches, size_t channels, size_t hei
                 g_launches.fetch_add(1);
                 CUDA_TRY(cudaGetLastError());
                 const long long wtotal = static_cast<long long>(num_kernels) * kb2 * 64;
-                cl_pack_small_filters_kernel<<<static_cast<unsigned>(std::min<long long>((wtotal + 255) / 256, 8ll * st->num_sms)), 256, 0, cs>>>(
+                CUDA_TRY(launch_dependent(cl_pack_small_filters_kernel, static_cast<unsigned>(std::min<long long>((wtotal + 255) / 256, 8ll * st->num_sms)), 256, 0, cs,
                     static_cast<const uint16_t*>(w), wpk, static_cast<int>(num_kernels), static_cast<int>(channels),
-                    static_cast<int>(kernel_h), static_cast<int>(kernel_w), static_cast<int>(kb2), static_cast<int>(swl));
+                    static_cast<int>(kernel_h), static_cast<int>(kernel_w), static_cast<int>(kb2), static_cast<int>(swl)));
                 g_launches.fetch_add(1);
                 CUDA_TRY(cudaGetLastError());
                 sp.xp = reinterpret_cast<const char*>(xp);
@@ -2356,9 +2385,9 @@ int dlf_b200_conv2d_fused(int dtype, size_t batches, size_t channels, size_t hei
                 g_launches.fetch_add(1);
                 CUDA_TRY(cudaGetLastError());
                 const long long wtotal = static_cast<long long>(num_kernels) * channels;
-                cl_pack_filters_kernel<<<static_cast<unsigned>(std::min<long long>((wtotal + 255) / 256, 8ll * st->num_sms)), 256, 0, cs>>>(
+                CUDA_TRY(launch_dependent(cl_pack_filters_kernel, static_cast<unsigned>(std::min<long long>((wtotal + 255) / 256, 8ll * st->num_sms)), 256, 0, cs,
                     static_cast<const uint16_t*>(w), wpk, static_cast<int>(num_kernels), static_cast<int>(channels),
-                    static_cast<int>(taps), static_cast<int>(channels));
+                    static_cast<int>(taps), static_cast<int>(channels)));
                 g_launches.fetch_add(1);
                 CUDA_TRY(cudaGetLastError());
                 hp_.xh = reinterpret_cast<const char*>(xh);
@@ -2496,9 +2525,9 @@ int dlf_b200_conv2d_fused(int dtype, size_t batches, size_t channels, size_t hei
                 if (!w_direct) {
                     const long long total = static_cast<long long>(num_kernels) * ck;
                     const unsigned blocks = static_cast<unsigned>(std::min<long long>((total + 255) / 256, 8ll * st->num_sms));
-                    cl_pack_filters_kernel<<<blocks, 256, 0, cs>>>( static_cast<const uint16_t*>(w), wp,
+                    CUDA_TRY(launch_dependent(cl_pack_filters_kernel, blocks, 256, 0, cs, static_cast<const uint16_t*>(w), wp,
                                               static_cast<int>(num_kernels), static_cast<int>(channels),
-                                              static_cast<int>(taps), static_cast<int>(ck));
+                                              static_cast<int>(taps), static_cast<int>(ck)));
                     g_launches.fetch_add(1);
                     CUDA_TRY(cudaGetLastError());
                 }

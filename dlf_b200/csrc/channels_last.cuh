@@ -15,10 +15,14 @@
 //       the filter bank with k ordered (tap, channel), Ck = C rounded up to the 64-channel
 //       k-block, zero-padded, so that one k-block is one tap's channel block.
 //
+// The filter pack needs nothing of the activation pack before it in the stream: as its programmatic dependent it
+// runs beside it, and waits for it at its end, so that whatever follows the filter pack follows both.
 // Both are bound by memory traffic: |X| read + |X'| written, a few MB for the filters.
 // X' must be 16-byte aligned (it is the base of a tensor map and written with 16-byte stores).
 #pragma once
 #include <cstdint>
+
+#include "ptx.cuh"
 
 namespace dlfb200 {
 
@@ -47,6 +51,7 @@ template <int MODE>
 __global__ void __launch_bounds__(256)
     cl_pack_activations_kernel(const uint16_t* __restrict__ x, uint16_t* __restrict__ xp, int C, long long plane,
                                int W, int OH, int OW, int sh, int sw, int Cp, long long total) {
+    ptx::launch_dependents();
     __shared__ __align__(16) uint16_t tile[kClTile][kClTile + 8];  // 144-byte rows: ldmatrix rows fall in distinct banks
     const int t = threadIdx.x;
     const int p0 = blockIdx.x * kClTile;
@@ -164,6 +169,7 @@ __global__ void __launch_bounds__(256)
 // L1) and land in W' one tap plane apart, consecutive threads writing consecutive channels
 __global__ void cl_pack_filters_kernel(const uint16_t* __restrict__ w, uint16_t* __restrict__ wp, int Cout, int C,
                                        int taps, int Ck) {
+    ptx::launch_dependents();
     const long long total = static_cast<long long>(Cout) * Ck;
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
          i += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -174,6 +180,7 @@ __global__ void cl_pack_filters_kernel(const uint16_t* __restrict__ w, uint16_t*
         for (int tap = 0; tap < taps; ++tap)
             dst[static_cast<long long>(tap) * Ck] = c < C ? src[tap] : static_cast<uint16_t>(0);
     }
+    ptx::wait_for_dependencies();
 }
 
 // Filters over at most 4 input channels (an RGB stem). With so few channels a filter tap is 8
@@ -195,6 +202,7 @@ __global__ void cl_pack_filters_kernel(const uint16_t* __restrict__ w, uint16_t*
 __global__ void __launch_bounds__(256)
     cl_pack_small_activations_kernel(const uint16_t* __restrict__ x, uint4* __restrict__ xp, int C, int H, int W,
                                      int J, int OWp, int sw, int rstep, int pad_t, int pad_l, long long total) {
+    ptx::launch_dependents();
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
          i += static_cast<long long>(gridDim.x) * blockDim.x) {
         const int ii = static_cast<int>(i % OWp);
@@ -224,6 +232,7 @@ __global__ void __launch_bounds__(256)
 // one thread per element of W'' (Cout, KB, 64)
 __global__ void cl_pack_small_filters_kernel(const uint16_t* __restrict__ w, uint16_t* __restrict__ wp, int Cout,
                                              int C, int KH, int KW, int KB, int sw) {
+    ptx::launch_dependents();
     const long long total = static_cast<long long>(Cout) * KB * 64;
     const int tpp = 8 / sw;  // taps per phase
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
@@ -239,6 +248,7 @@ __global__ void cl_pack_small_filters_kernel(const uint16_t* __restrict__ w, uin
         if (kh < KH && kw < KW && ch < C) v = w[((co * C + ch) * KH + kh) * KW + kw];
         wp[i] = v;
     }
+    ptx::wait_for_dependencies();
 }
 
 }  // namespace dlfb200

@@ -403,6 +403,11 @@ __global__ void __launch_bounds__(PAIR ? kThreadsPair : (USE_TMA ? tma_threads(E
         ptx::tma_prefetch_desc(&tmA);
         ptx::tma_prefetch_desc(&tmB);
     }
+    // The launch is a programmatic dependent of the kernel before it (launch() in api.cu): everything above ran
+    // beside that kernel's last tiles; nothing it may have written is touched before this.
+    // (forward of 256 images: 4092 -> 4063 us)
+    ptx::launch_dependents();
+    ptx::wait_for_dependencies();
     ptx::tc_fence_before();
     __syncthreads();
     if constexpr (PAIR) ptx::cluster_sync();  // the peer's barriers exist before anything remote happens

@@ -60,6 +60,7 @@ struct HaloParams {
 __global__ void __launch_bounds__(256)
     halo_pack_activations_kernel(const uint16_t* __restrict__ x, uint4* __restrict__ xh, int C, int H, int W, int Hp,
                                  int Wp, int pad_t, int pad_l, long long total) {
+    ptx::launch_dependents();
     const long long plane = static_cast<long long>(H) * W;
     const int CG = C / 8;
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
