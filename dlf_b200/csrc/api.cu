@@ -3265,6 +3265,18 @@ int dlf_b200_pool_nhwc(int dtype, int average, int count_include_pad, size_t bat
     g.count_include_pad = count_include_pad ? 1 : 0;
     g.total = total;
     cudaStream_t cs = static_cast<cudaStream_t>(stream);
+    // a window that is the whole image goes to the kernel whose warps share its pixels
+    const long long groups = static_cast<long long>(batches) * ((g.C8 + 31) / 32);
+    if (output_h == 1 && output_w == 1 && pad_top == 0 && pad_left == 0 && kernel_h == height && kernel_w == width &&
+        height * width >= 8 && height * width < INT_MAX && groups < INT_MAX) {
+        if (fmt == FMT_F16)
+            pool_nhwc_global_kernel<OUT_F16><<<static_cast<unsigned>(groups), 256, 0, cs>>>(static_cast<const uint4*>(x), static_cast<uint4*>(y), g);
+        else
+            pool_nhwc_global_kernel<OUT_BF16><<<static_cast<unsigned>(groups), 256, 0, cs>>>(static_cast<const uint4*>(x), static_cast<uint4*>(y), g);
+        g_launches.fetch_add(1);
+        CUDA_TRY(cudaGetLastError());
+        return kSuccess;
+    }
     if (fmt == FMT_F16)
         pool_nhwc_kernel<OUT_F16><<<blocks, 256, 0, cs>>>(static_cast<const uint4*>(x), static_cast<uint4*>(y), g);
     else

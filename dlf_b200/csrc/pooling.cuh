@@ -428,4 +428,53 @@ __global__ void __launch_bounds__(256) pool_nhwc_kernel(const uint4* __restrict_
     }
 }
 
+// The same pooling over a window that is the whole image (global pooling: one output pixel, no padding). One
+// thread per 8 channels walked all pixels alone, each load waiting for the one before: 18.8 us for one image of
+// 2048 x 7 x 7, 31 us for 256 (1.6 TB/s). Here a block is 32 channel groups x 8 warps, warp w takes pixels w,
+// w + 8, ... with four loads in flight, and the eight partial results meet in shared memory in warp order.
+// Now 3.0 and 10.9 us (4.8 TB/s).
+template <int OUT>
+__global__ void __launch_bounds__(256) pool_nhwc_global_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, const PoolNhwc p) {
+    static_assert(OUT == OUT_F16 || OUT == OUT_BF16, "16-bit types");
+    using T = typename std::conditional<OUT == OUT_F16, __half, __nv_bfloat16>::type;
+    __shared__ float part[8][8][33];  // [warp][channel of the group][lane]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int groups = (p.C8 + 31) / 32;
+    const long long img = blockIdx.x / groups;
+    const int cg = (blockIdx.x - static_cast<int>(img) * groups) * 32 + lane;
+    const int pixels = p.H * p.W;
+    float acc[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[e] = p.average ? 0.0f : PoolType<T>::lowest();
+    if (cg < p.C8) {
+        const uint4* at = x + img * pixels * p.C8 + cg;
+#pragma unroll 4
+        for (int i = warp; i < pixels; i += 8) {
+            const uint4 u = at[static_cast<long long>(i) * p.C8];
+            const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                float2 f;
+                if constexpr (OUT == OUT_F16) f = __half22float2(*reinterpret_cast<const __half2*>(&w[g]));
+                else f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[g]));
+                acc[2 * g] = p.average ? acc[2 * g] + f.x : fmaxf(acc[2 * g], f.x);
+                acc[2 * g + 1] = p.average ? acc[2 * g + 1] + f.y : fmaxf(acc[2 * g + 1], f.y);
+            }
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) part[warp][e][lane] = acc[e];
+    __syncthreads();
+    // warp e finishes channel e of every group
+    float v = part[0][warp][lane];
+#pragma unroll
+    for (int k = 1; k < 8; ++k) v = p.average ? v + part[k][warp][lane] : fmaxf(v, part[k][warp][lane]);
+    if (p.average) v = v / static_cast<float>(pixels);
+    if (cg < p.C8) {
+        T* out = reinterpret_cast<T*>(y) + (img * p.C8 + cg) * 8 + warp;
+        if constexpr (OUT == OUT_F16) *out = __float2half_rn(v);
+        else *out = __float2bfloat16_rn(v);
+    }
+}
+
 }  // namespace dlfb200

@@ -161,3 +161,22 @@ def test_triangular_solve_with_a_zero_and_an_infinite_pivot(lib):
             T.view(-1), 0, n, B.view(-1), 0, 3)
     got = B.cpu()
     assert torch.isinf(got[5, 0]) and torch.isnan(got[5, 1]) and bool((got[:5] == 1.0).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16], ids=["f16", "bf16"])
+@pytest.mark.parametrize("shape", [(1, 2048, 7, 7), (3, 8, 2, 4), (2, 264, 3, 3), (2, 40, 33, 5)])
+def test_global_pooling_between_channels_last_tensors(lib, dtype, shape):
+    """pool_nhwc_global_kernel: channel groups that do not fill a warp, more and fewer pixels than warps."""
+    from dlf_b200 import gdnn
+    n, c, h, w = shape
+    X = _round_to(np.random.default_rng(c).normal(size=shape), dtype)
+    Xn = torch.from_numpy(X).to(dtype).cuda().permute(0, 2, 3, 1).contiguous()
+    for average in (True, False):
+        Y = torch.empty((n, 1, 1, c), dtype=dtype, device="cuda")
+        gdnn.pool_nhwc(Xn, Y, gdnn.Filter2D(shape, h, w).strides(h, w), average=average)
+        got = Y.float().cpu().numpy().reshape(n, c)
+        ref = oracle.global_pool(X, "avg" if average else "max", wide=True).reshape(n, c)
+        if average:
+            assert max_rel(got, ref) <= HALF_TOL
+        else:
+            assert np.array_equal(got, ref)
