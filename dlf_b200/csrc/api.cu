@@ -1307,7 +1307,8 @@ int launch(const Problem& q_in, cudaStream_t stream, DeviceState* preset = nullp
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
-    cfg.numAttrs = q_in.out_nchw != 0 || q_in.a_cl != 0 || total <= 2ll * st->num_sms ? 1 : 0;
+    p.dependent = q_in.out_nchw != 0 || q_in.a_cl != 0 || total <= 2ll * st->num_sms ? 1 : 0;
+    cfg.numAttrs = p.dependent ? 1 : 0;
     if (use_tma) {
 #define DLF_TMA_LAUNCH(ESETS)                                                                                      \
         cfg.blockDim = dim3(tma_threads(ESETS), 1, 1);                                                             \

@@ -172,6 +172,7 @@ struct Params {
                  // epilogue of the TMEM-operand kernel is skipped, 0x100 pooling always takes the
                  // plain one-thread-per-output kernel (results stay valid), 0x4000 no programmatic
                  // dependent launch after the filter-packing grid (results stay valid)
+    int dependent;  // the launch is a programmatic dependent of the kernel before it
 };
 
 struct PixelEntry {  // one output pixel of the current tile (implicit im2col operand)
@@ -403,11 +404,13 @@ __global__ void __launch_bounds__(PAIR ? kThreadsPair : (USE_TMA ? tma_threads(E
         ptx::tma_prefetch_desc(&tmA);
         ptx::tma_prefetch_desc(&tmB);
     }
-    // The launch is a programmatic dependent of the kernel before it (launch() in api.cu): everything above ran
-    // beside that kernel's last tiles; nothing it may have written is touched before this.
+    // A programmatic dependent of the kernel before it (launch() in api.cu) has set up its barriers, tensor memory and
+    // tensor maps beside that kernel's last tiles; nothing it may have written is touched before this.
     // (forward of 256 images: 4092 -> 4063 us)
-    ptx::launch_dependents();
-    ptx::wait_for_dependencies();
+    if (p.dependent) {
+        ptx::launch_dependents();
+        ptx::wait_for_dependencies();
+    }
     ptx::tc_fence_before();
     __syncthreads();
     if constexpr (PAIR) ptx::cluster_sync();  // the peer's barriers exist before anything remote happens
