@@ -149,10 +149,11 @@ constexpr int kTrsmOrder = 1024;   // unknowns one launch solves; longer systems
 constexpr int kTrsmThreads = 512;
 constexpr int kTrsmRowWarps = kTrsmThreads / 32 - 3;
 constexpr int kTrsmTileLd = 36;  // floats between the lines of a staged 32 x 32 tile (16-byte aligned lines)
+constexpr int kTrsmTurn = 64 * 20;  // floats of a row warp's transposition buffer: 64 lines of 16 + 4 or 32 of 32 + 4
 
 // dynamic shared memory of l3_trsm_kernel: the CTA's right-hand sides, then a transposition buffer per row warp
 constexpr size_t trsm_smem_bytes(int q, int columns, bool eq_contiguous) {
-    return static_cast<size_t>((q + 31) / 32 * 32) * columns * 4 + (eq_contiguous ? 0 : kTrsmRowWarps * 32 * 33 * 4);
+    return static_cast<size_t>((q + 63) / 64 * 64) * columns * 4 + (eq_contiguous ? 0 : kTrsmRowWarps * kTrsmTurn * 4);
 }
 
 // Substitution, whole: q <= kTrsmOrder unknowns of `nsys` independent systems, C systems per CTA, which stay
@@ -163,14 +164,15 @@ constexpr size_t trsm_smem_bytes(int q, int columns, bool eq_contiguous) {
 // The unused triangle, and the diagonal of a unit-triangular matrix, are not read.
 //
 // What bounds it is the chain of unknowns, so the block of 32 unknowns at hand is all that warp 0 works on:
-// it takes the newest 32 solved unknowns out of the next 32 equations (lane = equation) and solves those (lane =
-// system, 32 values in registers, the products of a solved unknown are independent of one another), while
-// warps 1 and 2 fetch the two coefficient tiles warp 0 needs in the step after and the other 13 warps take the newest
-// unknowns out of all later equations, each with its next tile of coefficients already on the way. One barrier
+// lane = equation, it takes the newest 32 solved unknowns out of the next 32 equations and solves those, the systems
+// side by side to cover the latency of the shuffles (with many systems lane = system), while warps
+// 1 and 2 fetch the two coefficient tiles warp 0 needs two steps later and the other 13 warps take the newest
+// unknowns out of all later equations (the solved unknowns come from shared memory, 16 bytes a lane,
+// which is what sets their pace), each with its next 32 coefficients already on the way. One barrier
 // per 32 unknowns. A quotient is a product with the reciprocal and one correction step (12 clocks of latency
 // instead of a division's); a block with a result that is not finite is solved again with divisions.
-// Measured (fp32, 1024 unknowns x 512 systems): 947 us for 16 launches of one thread per system and 15 products
-// between them, 135 us now; 512 x 512 52-56 us, 128 x 512 13 us, 48 x 48 6 us.
+// Measured (fp32): 1024 unknowns x 512 systems 947 us in 16 launches of one thread per system and 15 products between
+// them, now 93 (equations contiguous) to 119 us (unknowns); 512 x 512 37 to 45, 128 x 512 11 to 13, 48 x 48 6 us.
 template <typename T, bool EQC, int C>
 __global__ void __launch_bounds__(kTrsmThreads, 1)
     l3_trsm_kernel(const T* __restrict__ base, long long se, long long sv, int unit, int q, T* __restrict__ b,
@@ -182,7 +184,15 @@ __global__ void __launch_bounds__(kTrsmThreads, 1)
     __shared__ float2 pivot[2][32];                           // diagonal element and its reciprocal
     const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
-    const int blocks = (q + 31) / 32;
+    const int blocks = (q + 31) / 32, rows = (q + 63) / 64 * 64;
+    // Up to 8 systems: warp 0 solves them by shuffles, a row lane takes two equations. With more, a lane of warp 0
+    // solves one system and a row lane has one equation (2500 x 2500: 684 us by shuffles and two
+    // equations a lane, 548 so).
+    constexpr bool kFew = C <= 8;
+    constexpr int RPL = kFew ? 2 : 1;        // equations per row lane
+    constexpr int UW = 32 / RPL;             // unknowns at a time
+    constexpr int kUnroll = C <= 4 ? 8 : 4;  // short loops: unrolled in full, warp 0's code is fetched again every step
+    const int groups = (q + 32 * RPL - 1) / (32 * RPL);
     float* R = trsm_smem;  // [equation][C]
     const int sys0 = blockIdx.x * C;
 
@@ -218,53 +228,100 @@ __global__ void __launch_bounds__(kTrsmThreads, 1)
         }
         d = !unit && p0 + lane < q ? l3_load(base + (p0 + lane) * (se + sv)) : 1.0f;
     };
-    // equations p0 + lane lose the unknowns of block j; coef(i) = coefficient of unknown i in the lane's equation
-    auto eliminate = [&](int p0, int j, auto coef) {
-        float4 acc[C / 4];
-        float4* row = reinterpret_cast<float4*>(R + (p0 + lane) * C);
-#pragma unroll
-        for (int c = 0; c < C / 4; ++c) acc[c] = row[c];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-            const float k = -coef(i);
-            const float4* x = reinterpret_cast<const float4*>(R + (j * 32 + i) * C);
-#pragma unroll
-            for (int c = 0; c < C / 4; ++c) {
-                const float4 xv = x[c];
-                acc[c].x = fmaf(k, xv.x, acc[c].x);
-                acc[c].y = fmaf(k, xv.y, acc[c].y);
-                acc[c].z = fmaf(k, xv.z, acc[c].z);
-                acc[c].w = fmaf(k, xv.w, acc[c].w);
-            }
-        }
-#pragma unroll
-        for (int c = 0; c < C / 4; ++c) row[c] = acc[c];
+    auto fma4 = [](float4& a, float k, const float4& x) {
+        a.x = fmaf(k, x.x, a.x);
+        a.y = fmaf(k, x.y, a.y);
+        a.z = fmaf(k, x.z, a.z);
+        a.w = fmaf(k, x.w, a.w);
     };
-    auto solve_block = [&](int j) {  // warp 0
+    // warp 0: block j, with the unknowns of block j - 1 still in its equations (j > 0)
+    auto solve_block = [&](int j) {
         const float* tile = dia[j & 1];
         const float2* piv = pivot[j & 1];
-        float* col = R + j * 32 * C + min(lane, C - 1);
-        float a[32];
-        float worst = 0.0f;
+        float4* row = reinterpret_cast<float4*>(R + (j * 32 + lane) * C);
+        float4 acc[C / 4];
 #pragma unroll
-        for (int r = 0; r < 32; ++r) a[r] = col[r * C];
+        for (int c = 0; c < C / 4; ++c) acc[c] = row[c];
+        if (j > 0) {
+            const float* left = sub[j & 1];
+#pragma unroll kUnroll
+            for (int i = 0; i < 32; ++i) {
+                const float k = -left[i * kTrsmTileLd + lane];
+                const float4* x = reinterpret_cast<const float4*>(R + ((j - 1) * 32 + i) * C);
 #pragma unroll
-        for (int s = 0; s < 32; ++s) {
-            const float2 d = piv[s];
-            const float quot = a[s] * d.y;
-            const float x = fmaf(fmaf(-quot, d.x, a[s]), d.y, quot);
-            a[s] = x;
-            worst = fmaf(0.0f, x, worst);  // NaN from here on if x is not finite
-#pragma unroll
-            for (int g = (s + 1) / 4; g < 8; ++g) {
-                const float4 k = *reinterpret_cast<const float4*>(tile + s * kTrsmTileLd + g * 4);
-                if (g * 4 > s) a[g * 4] = fmaf(-k.x, x, a[g * 4]);
-                if (g * 4 + 1 > s) a[g * 4 + 1] = fmaf(-k.y, x, a[g * 4 + 1]);
-                if (g * 4 + 2 > s) a[g * 4 + 2] = fmaf(-k.z, x, a[g * 4 + 2]);
-                if (g * 4 + 3 > s) a[g * 4 + 3] = fmaf(-k.w, x, a[g * 4 + 3]);
+                for (int c = 0; c < C / 4; ++c) fma4(acc[c], k, x[c]);
             }
         }
-        if (__any_sync(0xffffffffu, worst != 0.0f)) {  // (NaN != 0)
+        bool redo;
+        if constexpr (kFew) {
+            const float2 d = piv[lane];
+            auto over = [&](float a) {
+                const float quot = a * d.y;
+                return fmaf(fmaf(-quot, d.x, a), d.y, quot);
+            };
+            float a[C];
+#pragma unroll
+            for (int c = 0; c < C / 4; ++c) {
+                a[4 * c] = acc[c].x;
+                a[4 * c + 1] = acc[c].y;
+                a[4 * c + 2] = acc[c].z;
+                a[4 * c + 3] = acc[c].w;
+            }
+            // (a lane's coefficients of its own and of later unknowns are zero: its right-hand sides stay)
+#pragma unroll kUnroll
+            for (int s = 0; s < 32; ++s) {
+                const float k = -tile[s * kTrsmTileLd + lane];
+#pragma unroll
+                for (int c = 0; c < C; ++c) a[c] = fmaf(k, __shfl_sync(0xffffffffu, over(a[c]), s), a[c]);
+            }
+            float check = 0.0f;
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                a[c] = over(a[c]);
+                check = fmaf(0.0f, a[c], check);  // NaN if a result is not finite
+            }
+            redo = __any_sync(0xffffffffu, check != 0.0f);
+            if (!redo) {
+#pragma unroll
+                for (int c = 0; c < C / 4; ++c) row[c] = make_float4(a[4 * c], a[4 * c + 1], a[4 * c + 2], a[4 * c + 3]);
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < C / 4; ++c) row[c] = acc[c];
+            __syncwarp();
+            float* col = R + j * 32 * C + min(lane, C - 1);
+            float a[32];
+            float check = 0.0f;
+#pragma unroll
+            for (int r = 0; r < 32; ++r) a[r] = col[r * C];
+#pragma unroll
+            for (int s = 0; s < 32; ++s) {
+                const float2 d = piv[s];
+                const float quot = a[s] * d.y;
+                const float x = fmaf(fmaf(-quot, d.x, a[s]), d.y, quot);
+                a[s] = x;
+                check = fmaf(0.0f, x, check);
+#pragma unroll
+                for (int g = (s + 1) / 4; g < 8; ++g) {
+                    const float4 k = *reinterpret_cast<const float4*>(tile + s * kTrsmTileLd + g * 4);
+                    if (g * 4 > s) a[g * 4] = fmaf(-k.x, x, a[g * 4]);
+                    if (g * 4 + 1 > s) a[g * 4 + 1] = fmaf(-k.y, x, a[g * 4 + 1]);
+                    if (g * 4 + 2 > s) a[g * 4 + 2] = fmaf(-k.z, x, a[g * 4 + 2]);
+                    if (g * 4 + 3 > s) a[g * 4 + 3] = fmaf(-k.w, x, a[g * 4 + 3]);
+                }
+            }
+            redo = __any_sync(0xffffffffu, check != 0.0f);
+            if (!redo && lane < C) {
+#pragma unroll
+                for (int r = 0; r < 32; ++r) col[r * C] = a[r];
+            }
+        }
+        if (redo) {
+            __syncwarp();
+#pragma unroll
+            for (int c = 0; c < C / 4; ++c) row[c] = acc[c];
+            __syncwarp();
+            float* col = R + j * 32 * C + min(lane, C - 1);
 #pragma unroll 1
             for (int s = 0; s < 32; ++s) {
                 const float x = col[s * C] / piv[s].x;
@@ -275,17 +332,16 @@ __global__ void __launch_bounds__(kTrsmThreads, 1)
                 }
                 __syncwarp();
             }
-        } else if (lane < C) {
-#pragma unroll
-            for (int r = 0; r < 32; ++r) col[r * C] = a[r];
         }
         __syncwarp();
     };
 
-    for (int id = threadIdx.x; id < blocks * 32 * C; id += kTrsmThreads) {
-        // threads run along the direction of b that is contiguous
-        const bool across = b_system == 1;
-        const int p = across ? id / C : id % (blocks * 32), t = across ? id % C : id / (blocks * 32);
+    // right-hand sides in and out; threads run along the direction of b that is contiguous
+    const int total = rows * C;
+    const bool across = b_system == 1;
+#pragma unroll 4
+    for (int id = threadIdx.x; id < total; id += kTrsmThreads) {
+        const int p = across ? id / C : id % rows, t = across ? id % C : id / rows;
         R[p * C + t] = p < q && sys0 + t < nsys ? alpha * l3_load(b + p * b_unknown + (sys0 + t) * b_system) : 0.0f;
     }
     // The two fetching warps run two steps ahead: what is stored for block j + 2 in step j was loaded during
@@ -295,9 +351,6 @@ __global__ void __launch_bounds__(kTrsmThreads, 1)
         solve_block(0);
         __syncthreads();
         for (int j = 0; j + 1 < blocks; ++j) {
-            const float* tile = sub[(j + 1) & 1];
-            eliminate((j + 1) * 32, j, [&](int i) { return tile[i * kTrsmTileLd + lane]; });
-            __syncwarp();
             solve_block(j + 1);
             __syncthreads();
         }
@@ -323,12 +376,10 @@ __global__ void __launch_bounds__(kTrsmThreads, 1)
         };
         load_dia(v, d, 0);
         put_dia(0);
-        if (blocks > 1) {
-            load_dia(v, d, 1);
-            put_dia(1);
-        }
-        if (blocks > 2) load_dia(v, d, 2);
+        if (blocks > 1) load_dia(v, d, 1);
         __syncthreads();
+        if (blocks > 1) put_dia(1);
+        if (blocks > 2) load_dia(v, d, 2);
         __syncthreads();
         for (int j = 0; j + 1 < blocks; ++j) {
             if (j + 2 < blocks) put_dia(j + 2);
@@ -336,40 +387,104 @@ __global__ void __launch_bounds__(kTrsmThreads, 1)
             __syncthreads();
         }
     } else {
+        // Groups of 32 * RPL equations, RPL per lane (32 apart): this warp's are g == w modulo kTrsmRowWarps. In step j it
+        // takes block j's unknowns, UW at a time, out of those of its equations that lie behind block j + 1.
+        constexpr int TLD = UW + 4;
         const int w = warp - 3;
-        float* turn = trsm_smem + blocks * 32 * C + w * 32 * 33;
-        // this warp's row tiles are p == w modulo kTrsmRowWarps; the first one not before block j + 2
-        auto first = [&](int j) { return j + 2 + (w + kTrsmRowWarps - (j + 2) % kTrsmRowWarps) % kTrsmRowWarps; };
+        float* turn = trsm_smem + total + w * kTrsmTurn;
+        auto first = [&](int j) {
+            const int g = (j + 2) / RPL;
+            return g + (w + kTrsmRowWarps - g % kTrsmRowWarps) % kTrsmRowWarps;
+        };
+        auto load_part = [&](float (&v)[32], int g, int j, int h) {
+            const int p0 = g * 32 * RPL, v0 = j * 32 + h * UW, lo = (j + 2) * 32;
+            if constexpr (EQC) {
+#pragma unroll
+                for (int k = 0; k < RPL; ++k) {
+                    const int p = p0 + 32 * k + lane;
+                    const bool inside = p >= lo && p < q;
+                    const T* at = base + p * se + v0 * sv;
+#pragma unroll
+                    for (int i = 0; i < UW; ++i) v[UW * k + i] = inside ? l3_load(at + i * sv) : 0.0f;
+                }
+            } else {
+                const int p1 = p0 + lane / UW;
+                const T* at = base + p1 * se + (v0 + lane % UW) * sv;
+#pragma unroll
+                for (int i = 0; i < 32; ++i) {
+                    const int p = p1 + RPL * i;
+                    v[i] = p >= lo && p < q ? l3_load(at + RPL * i * se) : 0.0f;
+                }
+            }
+        };
         float v[32], next[32];
-        int p = first(0);
-        if (p < blocks) load_tile(v, p * 32, 0);
+        int g = first(0), h = 0;
+        if (g < groups) load_part(v, g, 0, 0);
         __syncthreads();
         __syncthreads();
         for (int j = 0; j + 1 < blocks; ++j) {
-            while (p < blocks) {
-                const bool same = p + kTrsmRowWarps < blocks;
-                const int np = same ? p + kTrsmRowWarps : first(j + 1), nj = same ? j : j + 1;
-                if (np < blocks) load_tile(next, np * 32, nj * 32);
-                if constexpr (EQC) {
-                    eliminate(p * 32, j, [&](int i) { return v[i]; });
-                } else {
+            while (g < groups) {
+                // what comes next: the group's next unknowns, else the first ones of the next group or of the next step
+                const bool within = h + 1 < RPL;
+                const bool same = within || g + kTrsmRowWarps < groups;
+                const int nh = within ? h + 1 : 0;
+                const int ng = within ? g : (same ? g + kTrsmRowWarps : first(j + 1));
+                if (ng < groups) load_part(next, ng, same ? j : j + 1, nh);
+                float4 acc[RPL][C / 4];
+#pragma unroll
+                for (int k = 0; k < RPL; ++k) {
+                    const float4* row = reinterpret_cast<const float4*>(R + ((g * RPL + k) * 32 + lane) * C);
+#pragma unroll
+                    for (int c = 0; c < C / 4; ++c) acc[k][c] = row[c];
+                }
+                if constexpr (!EQC) {
                     __syncwarp();
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) turn[lane * 33 + i] = v[i];
+                    for (int i = 0; i < 32; ++i) turn[(RPL * i + lane / UW) * TLD + lane % UW] = v[i];
                     __syncwarp();
-                    eliminate(p * 32, j, [&](int i) { return turn[i * 33 + lane]; });
+#pragma unroll
+                    for (int k = 0; k < RPL; ++k) {
+#pragma unroll
+                        for (int i = 0; i < UW; i += 4) {
+                            const float4 e = *reinterpret_cast<const float4*>(turn + (32 * k + lane) * TLD + i);
+                            v[UW * k + i] = e.x;
+                            v[UW * k + i + 1] = e.y;
+                            v[UW * k + i + 2] = e.z;
+                            v[UW * k + i + 3] = e.w;
+                        }
+                    }
+                }
+                const float4* x = reinterpret_cast<const float4*>(R + (j * 32 + h * UW) * C);
+#pragma unroll
+                for (int i = 0; i < UW; ++i) {
+#pragma unroll
+                    for (int c = 0; c < C / 4; ++c) {
+                        const float4 xv = x[i * (C / 4) + c];
+#pragma unroll
+                        for (int k = 0; k < RPL; ++k) fma4(acc[k][c], -v[UW * k + i], xv);
+                    }
+                }
+                // (the first equations of a group may be block j + 1, which is warp 0's)
+#pragma unroll
+                for (int k = 0; k < RPL; ++k) {
+                    float4* row = reinterpret_cast<float4*>(R + ((g * RPL + k) * 32 + lane) * C);
+                    if (g * RPL + k >= j + 2) {
+#pragma unroll
+                        for (int c = 0; c < C / 4; ++c) row[c] = acc[k][c];
+                    }
                 }
 #pragma unroll
                 for (int i = 0; i < 32; ++i) v[i] = next[i];
-                p = np;
+                g = ng;
+                h = nh;
                 if (!same) break;
             }
             __syncthreads();
         }
     }
-    for (int id = threadIdx.x; id < blocks * 32 * C; id += kTrsmThreads) {
-        const bool across = b_system == 1;
-        const int p = across ? id / C : id % (blocks * 32), t = across ? id % C : id / (blocks * 32);
+#pragma unroll 4
+    for (int id = threadIdx.x; id < total; id += kTrsmThreads) {
+        const int p = across ? id / C : id % rows, t = across ? id % C : id / rows;
         if (p < q && sys0 + t < nsys) b[p * b_unknown + (sys0 + t) * b_system] = l3_make<T>(R[p * C + t]);
     }
 }

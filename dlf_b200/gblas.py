@@ -440,26 +440,35 @@ def syrk(layout, triangle, a_transpose, n, k, alpha, a_buffer, a_offset, a_ld, b
     _check(rc)
 
 
-def _triangular(fn_name, routine, layout, side, triangle, a_transpose, diagonal, m, n, alpha, a_buffer, a_offset,
-                a_ld, b_buffer, b_offset, b_ld, queue, event):
-    prec = precision_of(b_buffer)
-    if a_buffer.dtype != b_buffer.dtype:
+def _triangular(fn_name, routine, layout, side, triangle, a_transpose, diagonal, m, n, alpha, a, a_ld, b, b_ld, queue=None,
+                event=None):
+    prec = precision_of(b)
+    if a.dtype != b.dtype:
         raise BLASError(StatusCode.kInvalidValue)
     if m == 0 or n == 0:
         raise BLASError(StatusCode.kInvalidDimension)
     ka = m if int(side) == Side.Left else n
     row = int(layout) == Layout.RowMajor
-    _test_matrix(ka, ka, a_buffer, a_offset, a_ld, StatusCode.kInvalidLeadDimA, StatusCode.kInsufficientMemoryA)
+    _test_matrix(ka, ka, a, a.offset, a_ld, StatusCode.kInvalidLeadDimA, StatusCode.kInsufficientMemoryA)
     one, two = (n, m) if row else (m, n)
-    _test_matrix(one, two, b_buffer, b_offset, b_ld, StatusCode.kInvalidLeadDimB, StatusCode.kInsufficientMemoryB)
-    al = _scalar(alpha, b_buffer.dtype)
-    s, sp = _stream(queue)
-    ws = _level3_workspace(routine, b_buffer, m, n, s)
+    _test_matrix(one, two, b, b.offset, b_ld, StatusCode.kInvalidLeadDimB, StatusCode.kInsufficientMemoryB)
+    al = _scalar(alpha, b.dtype)
+    if not (a.is_cuda and b.is_cuda):
+        raise BLASError(StatusCode.kInvalidMatrixA)
+    L = lib()
+    handle = _raw_stream(queue)
+    need = L.dlf_b200_level3_workspace_bytes(routine, int(prec), m, n)
+    ws = None
+    if need:
+        ws = torch.empty(int(need), dtype=torch.uint8, device=b.device)
+        if queue is not None:
+            ws.record_stream(queue)  # read by work queued on a stream that may not be the allocator's
     if event is not None:
+        s = queue if queue is not None else torch.cuda.current_stream()
         event.start.record(s)
-    rc = getattr(lib(), fn_name)(int(prec), int(layout), int(side), int(triangle), int(a_transpose), int(diagonal),
-                                 m, n, ctypes.byref(al), _ptr(a_buffer, a_offset), a_ld, _ptr(b_buffer, b_offset),
-                                 b_ld, ctypes.c_void_p(ws.data_ptr()), ws.numel(), sp)
+    rc = getattr(L, fn_name)(int(prec), int(layout), int(side), int(triangle), int(a_transpose), int(diagonal), m, n,
+                             ctypes.byref(al), a.address, a_ld, b.address, b_ld,
+                             ws.data_ptr() if ws is not None else None, ws.numel() if ws is not None else 0, handle)
     if event is not None:
         event.end.record(s)
     _check(rc)
@@ -468,13 +477,13 @@ def _triangular(fn_name, routine, layout, side, triangle, a_transpose, diagonal,
 def trmm(layout, side, triangle, a_transpose, diagonal, m, n, alpha, a_buffer, a_offset, a_ld, b_buffer, b_offset,
          b_ld, queue=None, event=None):
     """B = alpha*op(T)*B (Left) or alpha*B*op(T) (Right), in place (gpgpu::blas::trmm, gblas.h:570-577)."""
-    _triangular("dlf_b200_trmm", _TRMM, layout, side, triangle, a_transpose, diagonal, m, n, alpha, a_buffer,
-                a_offset, a_ld, b_buffer, b_offset, b_ld, queue, event)
+    _triangular("dlf_b200_trmm", _TRMM, layout, side, triangle, a_transpose, diagonal, m, n, alpha,
+                _buffer_operand(a_buffer, a_offset), a_ld, _buffer_operand(b_buffer, b_offset), b_ld, queue, event)
 
 
 def trsm(layout, side, triangle, a_transpose, diagonal, m, n, alpha, a_buffer, a_offset, a_ld, b_buffer, b_offset,
          b_ld, queue=None, event=None):
     """Solves op(T)*X = alpha*B (Left) or X*op(T) = alpha*B (Right); X overwrites B
     (gpgpu::blas::trsm, gblas.h:579-586)."""
-    _triangular("dlf_b200_trsm", _TRSM, layout, side, triangle, a_transpose, diagonal, m, n, alpha, a_buffer,
-                a_offset, a_ld, b_buffer, b_offset, b_ld, queue, event)
+    _triangular("dlf_b200_trsm", _TRSM, layout, side, triangle, a_transpose, diagonal, m, n, alpha,
+                _buffer_operand(a_buffer, a_offset), a_ld, _buffer_operand(b_buffer, b_offset), b_ld, queue, event)

@@ -304,8 +304,12 @@ def _triangular(name, side, uplo, transA, diag, A, B, alpha, backend):
     if A.stride(1) != 1:
         raise ShapeError(name + ": A must be row-major")
     C = B.contiguous().clone()  # the reference copies B into the result and works in place (linalg.h:252-258)
-    getattr(be, name)(Layout.RowMajor, side, uplo, transA, diag, m, n, alpha, _flat(A), A.storage_offset(),
-                      A.stride(0), _flat(C), C.storage_offset(), C.stride(0))
+    if be is _gblas:
+        be._triangular("dlf_b200_" + name, be._TRMM if name == "trmm" else be._TRSM, Layout.RowMajor, side, uplo, transA, diag,
+                       m, n, alpha, be._view_operand(A), A.stride(0), be._view_operand(C), C.stride(0))
+    else:
+        getattr(be, name)(Layout.RowMajor, side, uplo, transA, diag, m, n, alpha, _flat(A), A.storage_offset(),
+                          A.stride(0), _flat(C), C.storage_offset(), C.stride(0))
     return C
 
 
