@@ -398,6 +398,7 @@ __global__ void __launch_bounds__(PAIR ? kThreadsPair : (USE_TMA ? tma_threads(E
         } else {
             ptx::tmem_alloc(ptx::smem_u32(&tmem_slot), tmem_cols);
             ptx::tmem_relinquish();
+            if (p.dependent) ptx::launch_dependents();  // (in this warp, with the tensor memory in hand: see ptx.cuh)
         }
     }
     if (USE_TMA && warp == kTmaWarp && lane == 0) {
@@ -407,10 +408,7 @@ __global__ void __launch_bounds__(PAIR ? kThreadsPair : (USE_TMA ? tma_threads(E
     // A programmatic dependent of the kernel before it (launch() in api.cu) has set up its barriers, tensor memory and
     // tensor maps beside that kernel's last tiles; nothing it may have written is touched before this.
     // (forward of 256 images: 4092 -> 4063 us)
-    if (p.dependent) {
-        ptx::launch_dependents();
-        ptx::wait_for_dependencies();
-    }
+    if (p.dependent) ptx::wait_for_dependencies();
     ptx::tc_fence_before();
     __syncthreads();
     if constexpr (PAIR) ptx::cluster_sync();  // the peer's barriers exist before anything remote happens

@@ -119,6 +119,7 @@ __global__ void __launch_bounds__(kF32Threads, 1)
         __syncwarp();
         ptx::tmem_alloc(ptx::smem_u32(&tmem_slot), 512u);
         ptx::tmem_relinquish();
+        ptx::launch_dependents();  // (in this warp, with the tensor memory in hand: see ptx.cuh)
     }
     if (warp == 12 && lane == 0) {
         ptx::tma_prefetch_desc(&tmA);
@@ -130,7 +131,6 @@ __global__ void __launch_bounds__(kF32Threads, 1)
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&tmem_slot);
     volatile int* abort_p = &abort_flag;
     const long long wait_limit = p.wait_limit;
-    ptx::launch_dependents();
     ptx::wait_for_dependencies();
     // the launch has 512 x 128 registers: 2 x 176 + 96 + 64 = 4 x 128
     if (warp < 8) asm volatile("setmaxnreg.inc.sync.aligned.u32 176;");

@@ -71,7 +71,6 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
     const int tn = (tile - b * per) / p.tiles_m, tm = tile - b * per - tn * p.tiles_m;
     const int m0 = tm * kBM, n0 = tn * kSplitBN;
 
-    ptx::launch_dependents();
     if (threadIdx.x == 0) {
         abort_flag = 0;
         for (int s = 0; s < p.stages; ++s) {
@@ -85,6 +84,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
         __syncwarp();
         ptx::tmem_alloc(ptx::smem_u32(&tmem_slot), 64u);
         ptx::tmem_relinquish();
+        ptx::launch_dependents();  // (in this warp, with the tensor memory in hand: see ptx.cuh)
     }
     if (warp == 4 && lane == 0) {
         ptx::tma_prefetch_desc(&tmA);

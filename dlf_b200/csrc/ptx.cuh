@@ -86,7 +86,10 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
 // ---------------------------------------------------------------- launches
 // Programmatic dependent launch: the next kernel of the stream may start (its CTAs wait below until this grid
 // has completed) / wait for the grids before this one.
-__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
+// The first thread of a CTA that gets here speaks for the CTA. In a kernel that allocates tensor memory that has
+// to be the allocating warp, behind its allocation: a dependent's CTA on the same SM could otherwise take the
+// tensor memory first and keep it while it waits for this grid, which would wait for the tensor memory.
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_dependencies() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // ---------------------------------------------------------------- fences

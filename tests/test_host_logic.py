@@ -136,3 +136,36 @@ def test_product_never_imports_the_oracle():
             if fn.endswith((".py", ".cu", ".cuh", ".h", ".hpp")):
                 text = open(os.path.join(dirpath, fn)).read()
                 assert "import oracle" not in text and "dlf_oracle" not in text, fn
+
+
+def _kernels(text):
+    """(name, body) of every __global__ function of a CUDA source, without comments."""
+    text = re.sub(r"//[^\n]*", "", text)
+    for m in re.finditer(r"__global__", text):
+        head = text.index("{", m.end())
+        name = re.findall(r"(\w+)\s*\(", text[m.end():head].replace("__launch_bounds__", ""))
+        depth, i = 1, head + 1
+        while depth:
+            depth += {"{": 1, "}": -1}.get(text[i], 0)
+            i += 1
+        yield [n for n in name if n.endswith("_kernel")][-1], text[head:i]
+
+
+def test_dependents_are_launched_by_the_warp_that_holds_the_tensor_memory():
+    """A kernel that allocates tensor memory may let the next kernel start only behind the allocation, and in
+    the warp that made it: the next kernel's CTA keeps what it allocates while it waits for this grid, so
+    one that got there first would stop both."""
+    csrc = os.path.join(ROOT, "dlf_b200", "csrc")
+    checked = []
+    for fn in sorted(os.listdir(csrc)):
+        for name, body in _kernels(open(os.path.join(csrc, fn)).read()):
+            if "tmem_alloc(" not in body or "launch_dependents" not in body:
+                continue
+            assert body.count("launch_dependents") == 1, name
+            at = body.index("launch_dependents")
+            allocated = body.rindex("tmem_alloc(", 0, at) if "tmem_alloc(" in body[:at] else None
+            assert allocated is not None, "%s starts its dependents before it allocates" % name
+            # no block closes in between: the same warp's branch
+            assert "}" not in body[allocated:at], "%s: another warp may start the dependents first" % name
+            checked.append(name)
+    assert checked == ["contraction_kernel", "contraction_f32_kernel", "contraction_split_kernel"]
