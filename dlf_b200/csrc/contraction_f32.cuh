@@ -224,27 +224,41 @@ __global__ void __launch_bounds__(kF32Threads, 1)
                 }
                 const uint32_t sA = smem0 + s * STAGE;
                 uint32_t hi[32], lo[32];
-                if (p.a.k_major) {
+                auto load_row = [&](uint32_t (&x)[32]) {
+                    if (p.a.k_major) {
 #pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        const uint4 u = ld_shared_v4(sA + L * 128u + ((c ^ (L & 7)) << 4));
-                        hi[4 * c + 0] = u.x;
-                        hi[4 * c + 1] = u.y;
-                        hi[4 * c + 2] = u.z;
-                        hi[4 * c + 3] = u.w;
+                        for (int c = 0; c < 8; ++c) {
+                            const uint4 u = ld_shared_v4(sA + L * 128u + ((c ^ (L & 7)) << 4));
+                            x[4 * c + 0] = u.x;
+                            x[4 * c + 1] = u.y;
+                            x[4 * c + 2] = u.z;
+                            x[4 * c + 3] = u.w;
+                        }
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < 32; ++k)
+                            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(x[k]) : "r"(sA + k * (kBM * 4) + L * 4) : "memory");
                     }
-                } else {
-#pragma unroll
-                    for (int k = 0; k < 32; ++k)
-                        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(hi[k]) : "r"(sA + k * (kBM * 4) + L * 4) : "memory");
-                }
+                };
+                load_row(hi);
+                // hi = x rounded to tf32 (half away from zero), lo = the rest, prepared for the truncation it meets in
+                // the tensor core: split_tf32 in integer arithmetic, which the issue slots of these four warps have more
+                // room for (4096^3 624 us with the conversions, 582 so). It holds for finite values only - the addition
+                // carries the NaN that arithmetic returns, 0x7fffffff, past the exponent into -0 - and any other value
+                // leaves a rest that is not finite: such a row is split again by the conversions.
+                float check = 0.0f;
 #pragma unroll
                 for (int k = 0; k < 32; ++k) {
-                    // hi = x rounded to tf32 (half away from zero); lo = the rest, prepared for the
-                    // truncation it meets in the tensor core
                     const float x = __uint_as_float(hi[k]);
                     hi[k] = (hi[k] + 0x1000u) & 0xffffe000u;
-                    lo[k] = __float_as_uint(x - __uint_as_float(hi[k])) + 0x1000u;
+                    const float rest = x - __uint_as_float(hi[k]);
+                    check = fmaf(0.0f, rest, check);  // NaN if the rest is infinite or NaN
+                    lo[k] = __float_as_uint(rest) + 0x1000u;
+                }
+                if (check != 0.0f) {
+                    load_row(hi);
+#pragma unroll
+                    for (int k = 0; k < 32; ++k) split_tf32(hi[k], hi[k], lo[k]);
                 }
                 __syncwarp();
                 if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&raw_empty[s]));

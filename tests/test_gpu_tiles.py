@@ -180,3 +180,72 @@ def test_global_pooling_between_channels_last_tensors(lib, dtype, shape):
             assert max_rel(got, ref) <= HALF_TOL
         else:
             assert np.array_equal(got, ref)
+
+
+# the NaN that CUDA arithmetic returns, the same with a sign, numpy's, one whose payload a truncation to tf32 drops
+NAN_BITS = [0x7fffffff, 0xffffffff, 0x7fc00000, 0x7f800001]
+
+
+def _nan(bits):
+    return np.array([bits], dtype=np.uint32).view(np.float32)[0]
+
+
+@pytest.mark.parametrize("bits", NAN_BITS, ids=hex)
+@pytest.mark.parametrize("width,m,n,k", [(64, 196, 260, 320), (128, 196, 260, 320), (192, 196, 260, 320), (0, 68, 196, 1028)])
+def test_nan_in_a_fp32_operand_stays_nan(lib, bits, width, m, n, k):
+    """contraction_f32_kernel, each tile width and tiles shared by a cluster: a NaN of any payload in either operand
+    reaches every output it contributes to, and no other."""
+    from dlf_b200 import gblas as gb
+    rng = np.random.default_rng(m + n + k)
+    lib.set_tuning(width, 0)
+    for ta in (False, True):
+        for tb in (False, True):
+            for side in "AB":
+                A = rng.uniform(-1, 1, (m, k)).astype(np.float32)
+                B = rng.uniform(-1, 1, (k, n)).astype(np.float32)
+                expected = np.zeros((m, n), dtype=bool)
+                if side == "A":
+                    A[5, 3] = A[130 % m, k - 1] = _nan(bits)
+                    expected[[5, 130 % m]] = True
+                else:
+                    B[3, 5] = B[k - 1, 130] = _nan(bits)
+                    expected[:, [5, 130]] = True
+                C = torch.zeros(m * n, device="cuda")
+                gb.gemm(gb.Layout.RowMajor, gb.Transpose.Trans if ta else gb.Transpose.NoTrans,
+                        gb.Transpose.Trans if tb else gb.Transpose.NoTrans, m, n, k, 1.0,
+                        torch.from_numpy(np.ascontiguousarray(A.T if ta else A)).cuda().view(-1), 0, m if ta else k,
+                        torch.from_numpy(np.ascontiguousarray(B.T if tb else B)).cuda().view(-1), 0, k if tb else n, 0.0, C, 0, n)
+                got = C.cpu().numpy().reshape(m, n)
+                assert np.array_equal(np.isnan(got), expected), (ta, tb, side)
+                ref = np.where(np.isnan(A), 0.0, A).astype(np.float64) @ np.where(np.isnan(B), 0.0, B).astype(np.float64)
+                assert rel_fro(got[~expected], ref[~expected]) <= FP32_TOL
+
+
+@pytest.mark.parametrize("bits", NAN_BITS, ids=hex)
+def test_nan_in_a_stack_of_fp32_products_stays_nan(lib, bits):
+    from dlf_b200 import tensor
+    A, B = torch.ones(3, 132, 64), torch.ones(3, 64, 68)
+    A.numpy()[1, 7, 9] = _nan(bits)
+    B.numpy()[2, 9, 65] = _nan(bits)
+    got = torch.isnan(tensor.matmul(A.cuda(), B.cuda(), torch.empty(3, 132, 68, device="cuda")).cpu())
+    expected = torch.zeros(3, 132, 68, dtype=torch.bool)
+    expected[1, 7] = True
+    expected[2, :, 65] = True
+    assert torch.equal(got, expected)
+
+
+@pytest.mark.parametrize("bits", NAN_BITS, ids=hex)
+@pytest.mark.parametrize("size,stride", [(8, 1), (7, 1), (8, 2)], ids=["planes of 16 bytes", "odd planes", "stride 2"])
+def test_nan_in_a_pointwise_fp32_convolution_stays_nan(lib, bits, size, stride):
+    """1x1 filters: a NaN pixel reaches that pixel of every channel, a NaN weight every pixel of its channel."""
+    from dlf_b200 import gdnn
+    f = gdnn.Filter2D((2, 72, size, size), (68, 72, 1, 1)).strides(stride, stride)
+    X, W = torch.ones(2, 72, size, size), torch.ones(68, 72, 1, 1)
+    X.numpy()[1, 70, 4, 6] = _nan(bits)
+    W.numpy()[66, 71] = _nan(bits)
+    Y = torch.empty(f.output_shape(), device="cuda")
+    gdnn.conv2d_filter(X.cuda(), W.cuda(), Y, f)
+    expected = torch.zeros(f.output_shape(), dtype=torch.bool)
+    expected[1, :, 4 // stride, 6 // stride] = True
+    expected[:, 66] = True
+    assert torch.equal(torch.isnan(Y.cpu()), expected)
