@@ -8,6 +8,7 @@ strides are in elements; ``queue`` is a ``torch.cuda.Stream`` (default: the curr
 ``Event*`` (gpgpu/src/gpgpu_cu.cpp:389-398). Errors raise :class:`BLASError` carrying the
 reference's ``StatusCode`` value. Every call goes through the C-ABI of libdlf_b200.so.
 """
+import contextlib
 import ctypes
 import enum
 import math
@@ -160,23 +161,37 @@ def _caller_scratch(device, nbytes):
     return buf
 
 
-def _gemm_workspace(device, queue, handle, nbytes, at_least):
-    """One scratch buffer per (device, stream), grown on demand; calls on a stream are ordered, so
-    they can share it. `handle` is the stream's handle, `queue` the stream (None = the current one).
-    A buffer of the caller's (`scratch`) need only hold `at_least`: the call makes do with it."""
-    own = _caller_scratch(device, at_least)
-    if own is not None:
-        return own
-    key = (device.index, handle)
-    buf = _GEMM_WORKSPACES.get(key)
-    if buf is None or buf.numel() < nbytes:
-        stream = queue if queue is not None else torch.cuda.current_stream()
-        if buf is not None:
+class _StreamScratch:
+    """The scratch buffer of one (device, stream), grown on demand. Calls queued on a stream are ordered, so they
+    can share it, but a call queues several kernels that hand data on in it: `lock` is held while it does, or another
+    thread's kernels on the same stream could come between them."""
+
+    __slots__ = ("lock", "buffer")
+
+    def __init__(self):
+        self.lock = threading.Lock()
+        self.buffer = None
+
+    def at_least(self, nbytes, device, queue):
+        """The buffer, with room for `nbytes`; `queue` is the stream (None = the current one). Needs the lock."""
+        buf = self.buffer
+        if buf is None or buf.numel() < nbytes:
+            stream = queue if queue is not None else torch.cuda.current_stream()
+            if buf is not None:
+                buf.record_stream(stream)  # work queued earlier may still read the old buffer
+            buf = torch.empty(int(nbytes), dtype=torch.uint8, device=device)
             buf.record_stream(stream)
-        buf = torch.empty(int(nbytes), dtype=torch.uint8, device=device)
-        buf.record_stream(stream)
-        _GEMM_WORKSPACES[key] = buf
-    return buf
+            self.buffer = buf
+        return buf
+
+
+def _stream_scratch(table, device, handle):
+    key = (device.index, handle)
+    entry = table.get(key)
+    return entry if entry is not None else table.setdefault(key, _StreamScratch())
+
+
+_NO_LOCK = contextlib.nullcontext()  # a call that has its scratch to itself, or none
 
 
 def _check(rc):
@@ -269,18 +284,24 @@ def _gemm(layout, a_transpose, b_transpose, m, n, k, alpha, a, a_ld, b, b_ld, be
     # 0 bytes = not useful
     need = L.dlf_b200_gemm_scratch_bytes(int(prec), int(layout), int(a_transpose), int(b_transpose), m, n, k,
                                          a.address, a_ld, b.address, b_ld)
-    ws = None
+    ws, entry = None, None
     if need:
         least = L.dlf_b200_gemm_workspace_bytes(int(prec), m, n, k) if getattr(_SCRATCH, "buffer", None) is not None else 0
-        ws = _gemm_workspace(c.device, queue, handle, need, least)
-    if event is not None:
-        s = queue if queue is not None else torch.cuda.current_stream()
-        event.start.record(s)
-    rc = L.dlf_b200_gemm_ex(int(prec), int(layout), int(a_transpose), int(b_transpose), m, n, k, ctypes.byref(al), a.address, a_ld,
-                            b.address, b_ld, ctypes.byref(be), c.address, c_ld,
-                            ws.data_ptr() if ws is not None else None, ws.numel() if ws is not None else 0, handle)
-    if event is not None:
-        event.end.record(s)
+        # (a buffer of the caller's need only hold `least`: the call makes do with it)
+        ws = _caller_scratch(c.device, least)
+        if ws is None:
+            entry = _stream_scratch(_GEMM_WORKSPACES, c.device, handle)
+    with entry.lock if entry is not None else _NO_LOCK:
+        if entry is not None:
+            ws = entry.at_least(need, c.device, queue)
+        if event is not None:
+            s = queue if queue is not None else torch.cuda.current_stream()
+            event.start.record(s)
+        rc = L.dlf_b200_gemm_ex(int(prec), int(layout), int(a_transpose), int(b_transpose), m, n, k, ctypes.byref(al), a.address, a_ld,
+                                b.address, b_ld, ctypes.byref(be), c.address, c_ld,
+                                ws.data_ptr() if ws is not None else None, ws.numel() if ws is not None else 0, handle)
+        if event is not None:
+            event.end.record(s)
     _check(rc)
 
 

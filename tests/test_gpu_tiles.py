@@ -249,3 +249,28 @@ def test_nan_in_a_pointwise_fp32_convolution_stays_nan(lib, bits, size, stride):
     expected[1, :, 4 // stride, 6 // stride] = True
     expected[:, 66] = True
     assert torch.equal(torch.isnan(Y.cpu()), expected)
+
+
+def test_unaligned_products_from_two_threads_on_one_stream(lib):
+    """Each call queues copies of its operands and a product that reads them, in scratch the stream's calls share."""
+    import threading
+    from dlf_b200 import tensor
+    g = torch.Generator().manual_seed(5)
+    operands = [(torch.rand(601, 515 + 2 * i, generator=g).cuda(), torch.rand(515 + 2 * i, 803, generator=g).cuda()) for i in range(2)]
+    wanted = [(a.double() @ b.double()).float() for a, b in operands]
+    results = [[torch.empty(601, 803, device="cuda") for _ in range(300)] for _ in range(2)]
+    torch.cuda.synchronize()
+
+    def work(i):
+        for y in results[i]:
+            tensor.matmul(*operands[i], y)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    for i in range(2):
+        for y in results[i]:
+            assert float((y - wanted[i]).norm() / wanted[i].norm()) <= FP32_TOL
