@@ -11,7 +11,7 @@ import ctypes
 import torch
 
 from . import lib
-from .gblas import BLASError, StatusCode, _caller_scratch, _check, _ptr, _stream, precision_of
+from .gblas import BLASError, StatusCode, _NO_LOCK, _caller_scratch, _check, _ptr, _stream, _stream_scratch, precision_of
 
 
 class Filter2D:
@@ -81,26 +81,9 @@ class Filter2D:
         return (self.batches, self.num_kernels, self.output_h, self.output_w)
 
 
+# Scratch for packed filter banks and channels-last copies, one buffer per (device, stream), grown on demand - the
+# role the context's temporary-buffer pool plays in the reference (gpgpu/src/gpgpu.cpp:189-214).
 _WORKSPACES = {}
-
-
-def _workspace(device, stream, nbytes):
-    """Scratch for the packed filter bank, one buffer per (device, stream), grown on demand - the
-    role the context's temporary-buffer pool plays in the reference (gpgpu/src/gpgpu.cpp:189-214).
-    Calls on one stream are ordered, so they can share it."""
-    own = _caller_scratch(device, nbytes)
-    if own is not None:
-        return own
-    key = (device.index, stream.cuda_stream)
-    buf = _WORKSPACES.get(key)
-    if buf is None or buf.numel() < nbytes:
-        if buf is not None:
-            # earlier convolutions queued on this stream may still read the old buffer
-            buf.record_stream(stream)
-        buf = torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=device)
-        buf.record_stream(stream)
-        _WORKSPACES[key] = buf
-    return buf
 
 
 def conv2d(batches, channels, height, width, output_h, output_w, num_kernels, group, kernel_h,
@@ -134,21 +117,26 @@ def conv2d(batches, channels, height, width, output_h, output_w, num_kernels, gr
     if activation not in (None, "relu"):
         raise BLASError(StatusCode.kInvalidValue)
     s, sp = _stream(queue)
-    ws = _workspace(result_buffer.device, s, lib().dlf_b200_conv2d_workspace_bytes(
+    need = lib().dlf_b200_conv2d_workspace_bytes(
         int(prec), batches, channels, height, width, output_h, output_w, num_kernels, group,
-        kernel_h, kernel_w))
-    if event is not None:
-        event.start.record(s)
+        kernel_h, kernel_w)
+    ws = _caller_scratch(result_buffer.device, need)
+    entry = _stream_scratch(_WORKSPACES, result_buffer.device, s.cuda_stream) if ws is None else None
     null = ctypes.c_void_p(0)
-    rc = lib().dlf_b200_conv2d_fused(
-        int(prec), batches, channels, height, width, output_h, output_w, num_kernels, group,
-        kernel_h, kernel_w, pad_top, pad_left, pad_bottom, pad_right, stride_h, stride_w,
-        dilation_h, dilation_w, _ptr(im_buffer), _ptr(kernel_buffer),
-        _ptr(bias) if bias is not None else null,
-        _ptr(residual) if residual is not None else null, 1 if activation == "relu" else 0,
-        _ptr(result_buffer), ctypes.c_void_p(ws.data_ptr()), ws.numel(), sp)
-    if event is not None:
-        event.end.record(s)
+    with entry.lock if entry is not None else _NO_LOCK:
+        if entry is not None:
+            ws = entry.at_least(max(need, 256), result_buffer.device, s)
+        if event is not None:
+            event.start.record(s)
+        rc = lib().dlf_b200_conv2d_fused(
+            int(prec), batches, channels, height, width, output_h, output_w, num_kernels, group,
+            kernel_h, kernel_w, pad_top, pad_left, pad_bottom, pad_right, stride_h, stride_w,
+            dilation_h, dilation_w, _ptr(im_buffer), _ptr(kernel_buffer),
+            _ptr(bias) if bias is not None else null,
+            _ptr(residual) if residual is not None else null, 1 if activation == "relu" else 0,
+            _ptr(result_buffer), ctypes.c_void_p(ws.data_ptr()), ws.numel(), sp)
+        if event is not None:
+            event.end.record(s)
     _check(rc)
 
 

@@ -1,4 +1,4 @@
-"""CPU suite: the device scratch the Python mirror hands to products, with a library that only records. What the calls
+"""CPU suite: the device scratch the Python mirror hands to products and convolutions, with a library that only records. What the calls
 queue on a stream hand on in that scratch must not be mixed with another thread's."""
 import threading
 import time
@@ -7,6 +7,7 @@ import pytest
 import torch
 
 from dlf_b200 import gblas as gb
+from dlf_b200 import gdnn
 
 
 class _Library:
@@ -22,8 +23,11 @@ class _Library:
     def dlf_b200_gemm_workspace_bytes(self, *args):
         return 16
 
+    def dlf_b200_conv2d_workspace_bytes(self, *args):
+        return self.need
+
     def dlf_b200_gemm_ex(self, *args):
-        ws, ws_bytes, stream = args[-3:]
+        ws, ws_bytes, stream = (getattr(a, "value", a) for a in args[-3:])
         with self.guard:
             self.inside[ws] = self.inside.get(ws, 0) + 1
             self.most = max(self.most, self.inside[ws])
@@ -32,6 +36,8 @@ class _Library:
         with self.guard:
             self.inside[ws] -= 1
         return 0
+
+    dlf_b200_conv2d_fused = dlf_b200_gemm_ex
 
 
 class _Stream:
@@ -52,7 +58,10 @@ def product(monkeypatch):
     def install(**kw):
         library = _Library(**kw)
         monkeypatch.setattr(gb, "lib", lambda: library)
+        monkeypatch.setattr(gdnn, "lib", lambda: library)
+        monkeypatch.setattr(gdnn, "_ptr", lambda buf: buf.data_ptr())
         monkeypatch.setattr(gb, "_GEMM_WORKSPACES", {})
+        monkeypatch.setattr(gdnn, "_WORKSPACES", {})
         monkeypatch.setattr(torch.Tensor, "record_stream", lambda self, stream: None)
         return library
 
@@ -64,17 +73,23 @@ def _call(handle):
              0.0, _Matrix(), 35, queue=_Stream(handle))
 
 
-def _threads(*handles):
-    ts = [threading.Thread(target=lambda h=h: [_call(h) for _ in range(5)]) for h in handles]
+def _convolve(handle):
+    f = gdnn.Filter2D((1, 4, 3, 3), (4, 4, 1, 1))
+    gdnn.conv2d_filter(torch.zeros(36), torch.zeros(16), torch.zeros(36), f, queue=_Stream(handle))
+
+
+def _threads(*handles, call=_call):
+    ts = [threading.Thread(target=lambda h=h: [call(h) for _ in range(5)]) for h in handles]
     for t in ts:
         t.start()
     for t in ts:
         t.join()
 
 
-def test_two_threads_on_one_stream_queue_one_after_the_other(product):
+@pytest.mark.parametrize("call", [_call, _convolve], ids=["product", "convolution"])
+def test_threads_on_one_stream_queue_one_after_the_other(product, call):
     library = product(need=1000, seconds=0.01)
-    _threads(7, 7, 7)
+    _threads(7, 7, 7, call=call)
     assert len(library.calls) == 15 and len({ws for ws, _, _ in library.calls}) == 1
     assert library.most == 1
 
