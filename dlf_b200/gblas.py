@@ -191,6 +191,15 @@ def _stream_scratch(table, device, handle):
     return entry if entry is not None else table.setdefault(key, _StreamScratch())
 
 
+_KEPT_BYTES = 64 << 20  # of a product's scratch: the partial sums of a K-split fit, copies of large operands do not
+
+
+def _passing_scratch(nbytes, device, queue):
+    """Scratch for one call, back with the allocator - in the order of the call's stream - when the call returns."""
+    with torch.cuda.stream(queue) if queue is not None else _NO_LOCK:
+        return torch.empty(int(nbytes), dtype=torch.uint8, device=device)
+
+
 _NO_LOCK = contextlib.nullcontext()  # a call that has its scratch to itself, or none
 
 
@@ -290,7 +299,10 @@ def _gemm(layout, a_transpose, b_transpose, m, n, k, alpha, a, a_ld, b, b_ld, be
         # (a buffer of the caller's need only hold `least`: the call makes do with it)
         ws = _caller_scratch(c.device, least)
         if ws is None:
-            entry = _stream_scratch(_GEMM_WORKSPACES, c.device, handle)
+            if need > _KEPT_BYTES:
+                ws = _passing_scratch(need, c.device, queue)
+            else:
+                entry = _stream_scratch(_GEMM_WORKSPACES, c.device, handle)
     with entry.lock if entry is not None else _NO_LOCK:
         if entry is not None:
             ws = entry.at_least(need, c.device, queue)

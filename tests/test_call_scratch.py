@@ -1,5 +1,6 @@
 """CPU suite: the device scratch the Python mirror hands to products and convolutions, with a library that only records. What the calls
 queue on a stream hand on in that scratch must not be mixed with another thread's."""
+import contextlib
 import threading
 import time
 
@@ -62,6 +63,8 @@ def product(monkeypatch):
         monkeypatch.setattr(gdnn, "_ptr", lambda buf: buf.data_ptr())
         monkeypatch.setattr(gb, "_GEMM_WORKSPACES", {})
         monkeypatch.setattr(gdnn, "_WORKSPACES", {})
+        monkeypatch.setattr(torch.cuda, "stream", lambda stream: contextlib.nullcontext())
+        monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
         monkeypatch.setattr(torch.Tensor, "record_stream", lambda self, stream: None)
         return library
 
@@ -119,3 +122,13 @@ def test_a_callers_scratch_needs_no_lock_and_only_what_the_plain_product_uses(pr
     assert library.calls == [(own.data_ptr(), 64, 1)] and not gb._GEMM_WORKSPACES
     with gb.scratch(torch.empty(8, dtype=torch.uint8)), pytest.raises(gb.BLASError):
         _call(1)
+
+
+def test_scratch_for_copies_of_large_operands_is_not_kept(product):
+    library = product(need=100 << 20)
+    _call(1)
+    assert library.calls[0][1] == 100 << 20
+    assert all(e.buffer is None for e in gb._GEMM_WORKSPACES.values())
+    library.need = 1000
+    _call(1)
+    assert [e.buffer.numel() for e in gb._GEMM_WORKSPACES.values()] == [1000]
