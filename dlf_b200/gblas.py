@@ -200,6 +200,10 @@ def _passing_scratch(nbytes, device, queue):
         return torch.empty(int(nbytes), dtype=torch.uint8, device=device)
 
 
+def _capturing():
+    return torch.cuda.is_current_stream_capturing()
+
+
 _NO_LOCK = contextlib.nullcontext()  # a call that has its scratch to itself, or none
 
 
@@ -299,7 +303,9 @@ def _gemm(layout, a_transpose, b_transpose, m, n, k, alpha, a, a_ld, b, b_ld, be
         # (a buffer of the caller's need only hold `least`: the call makes do with it)
         ws = _caller_scratch(c.device, least)
         if ws is None:
-            if need > _KEPT_BYTES:
+            # what is kept stays small, and is never part of a CUDA graph: a buffer that later calls replace must
+            # not be written by replays, and one from a graph's memory pool must not be handed to other calls
+            if need > _KEPT_BYTES or _capturing():
                 ws = _passing_scratch(need, c.device, queue)
             else:
                 entry = _stream_scratch(_GEMM_WORKSPACES, c.device, handle)

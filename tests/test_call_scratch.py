@@ -132,3 +132,15 @@ def test_scratch_for_copies_of_large_operands_is_not_kept(product):
     library.need = 1000
     _call(1)
     assert [e.buffer.numel() for e in gb._GEMM_WORKSPACES.values()] == [1000]
+
+
+@pytest.mark.parametrize("call,table", [(_call, lambda: gb._GEMM_WORKSPACES)], ids=["product"])
+def test_a_captured_call_neither_uses_nor_leaves_kept_scratch(product, monkeypatch, call, table):
+    library = product(need=1000)
+    call(1)
+    kept = [e.buffer for e in table().values()]
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    library.need = 2000
+    call(1)
+    assert library.calls[0][0] == kept[0].data_ptr() and library.calls[1][0] != kept[0].data_ptr()
+    assert [e.buffer for e in table().values()] == kept

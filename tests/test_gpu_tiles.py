@@ -274,3 +274,27 @@ def test_unaligned_products_from_two_threads_on_one_stream(lib):
     for i in range(2):
         for y in results[i]:
             assert float((y - wanted[i]).norm() / wanted[i].norm()) <= FP32_TOL
+
+
+def test_a_captured_unaligned_product_survives_larger_ones(lib):
+    """The scratch of a captured call belongs to its graph: later calls on the stream that need more of it must
+    not take away what the replays write."""
+    from dlf_b200 import tensor
+    g = torch.Generator().manual_seed(6)
+
+    def operands(m, n, k):
+        a, b = torch.rand(m, k, generator=g).cuda(), torch.rand(k, n, generator=g).cuda()
+        return a, b, torch.empty(m, n, device="cuda")
+
+    a, b, y = operands(601, 803, 515)
+    tensor.matmul(a, b, y)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        tensor.matmul(a, b, y)
+    large = operands(1601, 1603, 1605)
+    tensor.matmul(*large)
+    others = [torch.full((601 * 516 * 4,), 7, dtype=torch.uint8, device="cuda") for _ in range(16)]
+    y.zero_()
+    graph.replay()
+    assert float((y - a @ b).norm() / y.norm()) <= 2e-3  # (torch's product of fp32 matrices may use tf32)
+    assert all(bool((o == 7).all()) for o in others)
