@@ -195,9 +195,13 @@ _KEPT_BYTES = 64 << 20  # of a product's scratch: the partial sums of a K-split 
 
 
 def _passing_scratch(nbytes, device, queue):
-    """Scratch for one call, back with the allocator - in the order of the call's stream - when the call returns."""
+    """Scratch for one call, back with the allocator - in the order of the call's stream - when the call returns.
+    None if the device has no room for it: products run without, through slower loads."""
     with torch.cuda.stream(queue) if queue is not None else _NO_LOCK:
-        return torch.empty(int(nbytes), dtype=torch.uint8, device=device)
+        try:
+            return torch.empty(int(nbytes), dtype=torch.uint8, device=device)
+        except torch.OutOfMemoryError:
+            return None
 
 
 def _capturing():

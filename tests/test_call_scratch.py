@@ -144,3 +144,14 @@ def test_a_captured_call_neither_uses_nor_leaves_kept_scratch(product, monkeypat
     call(1)
     assert library.calls[0][0] == kept[0].data_ptr() and library.calls[1][0] != kept[0].data_ptr()
     assert [e.buffer for e in table().values()] == kept
+
+
+def test_a_product_runs_without_scratch_where_the_device_has_no_room(product, monkeypatch):
+    library = product(need=100 << 20)
+
+    def full(*args, **kw):
+        raise torch.OutOfMemoryError
+
+    monkeypatch.setattr(torch, "empty", full)
+    _call(1)
+    assert library.calls == [(None, 0, 1)]
