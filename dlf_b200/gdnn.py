@@ -11,7 +11,8 @@ import ctypes
 import torch
 
 from . import lib
-from .gblas import BLASError, StatusCode, _NO_LOCK, _caller_scratch, _check, _ptr, _stream, _stream_scratch, precision_of
+from .gblas import (BLASError, StatusCode, _NO_LOCK, _caller_scratch, _capturing, _check, _passing_scratch, _ptr, _stream,
+                    _stream_scratch, precision_of)
 
 
 class Filter2D:
@@ -120,8 +121,11 @@ def conv2d(batches, channels, height, width, output_h, output_w, num_kernels, gr
     need = lib().dlf_b200_conv2d_workspace_bytes(
         int(prec), batches, channels, height, width, output_h, output_w, num_kernels, group,
         kernel_h, kernel_w)
-    ws = _caller_scratch(result_buffer.device, need)
-    entry = _stream_scratch(_WORKSPACES, result_buffer.device, s.cuda_stream) if ws is None else None
+    ws, entry = _caller_scratch(result_buffer.device, need), None
+    if ws is None and _capturing():
+        ws = _passing_scratch(max(need, 256), result_buffer.device, queue)  # (as of a product: never kept scratch in a graph)
+    elif ws is None:
+        entry = _stream_scratch(_WORKSPACES, result_buffer.device, s.cuda_stream)
     null = ctypes.c_void_p(0)
     with entry.lock if entry is not None else _NO_LOCK:
         if entry is not None:
@@ -134,7 +138,8 @@ def conv2d(batches, channels, height, width, output_h, output_w, num_kernels, gr
             dilation_h, dilation_w, _ptr(im_buffer), _ptr(kernel_buffer),
             _ptr(bias) if bias is not None else null,
             _ptr(residual) if residual is not None else null, 1 if activation == "relu" else 0,
-            _ptr(result_buffer), ctypes.c_void_p(ws.data_ptr()), ws.numel(), sp)
+            _ptr(result_buffer), ctypes.c_void_p(ws.data_ptr()) if ws is not None else null,
+            ws.numel() if ws is not None else 0, sp)
         if event is not None:
             event.end.record(s)
     _check(rc)

@@ -134,7 +134,8 @@ def test_scratch_for_copies_of_large_operands_is_not_kept(product):
     assert [e.buffer.numel() for e in gb._GEMM_WORKSPACES.values()] == [1000]
 
 
-@pytest.mark.parametrize("call,table", [(_call, lambda: gb._GEMM_WORKSPACES)], ids=["product"])
+@pytest.mark.parametrize("call,table", [(_call, lambda: gb._GEMM_WORKSPACES), (_convolve, lambda: gdnn._WORKSPACES)],
+                         ids=["product", "convolution"])
 def test_a_captured_call_neither_uses_nor_leaves_kept_scratch(product, monkeypatch, call, table):
     library = product(need=1000)
     call(1)
