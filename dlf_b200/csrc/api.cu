@@ -376,6 +376,8 @@ struct Problem {
     int out_nchw = 0;
     long long cl_n = 0, cl_h = 0, cl_w = 0, cl_cp = 0;
     bool d_f32 = false;  // 16-bit operands with fp32 output (partial products of a K-split GEMM)
+    bool b_round = false;  // contraction_f32_kernel: both parts of operand B rounded (F32_B_ROUND)
+    const char* b_lo = nullptr;  // operand B as two matrices of tf32 values, laid out alike: b.base and this (F32_B_SPLIT)
     bool no_ts = false;  // convolution whose taps overflow the k table's 16/32-bit fields
 };
 
@@ -935,6 +937,7 @@ int launch_f32(const DeviceState& st, const Problem& q, cudaStream_t stream) {
     p.relu = q.relu;
     p.out_nchw = q.out_nchw;
     p.g = q.g;
+    p.b_parts = q.b_lo != nullptr ? F32_B_SPLIT : q.b_round ? F32_B_ROUND : F32_B_TRUNCATE;
     p.status = st.status;
     set_wait_policy(p, total);
     CUtensorMap tm_a, tm_b;
@@ -942,6 +945,13 @@ int launch_f32(const DeviceState& st, const Problem& q, cudaStream_t stream) {
     if (rc != kSuccess) return rc;
     rc = encode_map(st, &tm_b, q.b, 4, q.N, q.K, q.batch, bn);
     if (rc != kSuccess) return rc;
+    CUtensorMap tm_lo = tm_b;
+    if (q.b_lo != nullptr) {
+        GenOperand lo = q.b;
+        lo.base = q.b_lo;
+        rc = encode_map(st, &tm_lo, lo, 4, q.N, q.K, q.batch, bn);
+        if (rc != kSuccess) return rc;
+    }
 
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(split > 1 ? total * split : std::min<long long>(total, st.num_sms)), 1, 1);
@@ -962,7 +972,7 @@ int launch_f32(const DeviceState& st, const Problem& q, cudaStream_t stream) {
         std::fprintf(stderr, "dlf_b200: f32 launch bn=%d split=%d tiles=%lld stages=%d clusters 2:%d 3:%d 4:%d 8:%d\n", bn, split, total,
                      stages, st.max_f32_clusters[2], st.max_f32_clusters[3], st.max_f32_clusters[4], st.max_f32_clusters[8]);
     const auto kernel = nb == 1 ? contraction_f32_kernel<1> : nb == 2 ? contraction_f32_kernel<2> : contraction_f32_kernel<3>;
-    CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, p, tm_a, tm_b, split));
+    CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, p, tm_a, tm_b, tm_lo, split));
     g_launches.fetch_add(1);
     CUDA_TRY(cudaGetLastError());
     return kSuccess;
@@ -1106,7 +1116,7 @@ int launch(const Problem& q_in, cudaStream_t stream, DeviceState* preset = nullp
                          ((q.a_cl != 0 && !q.cl_swap) || tma_ok(q.a, q.es, q.M, q.K, q.batch)) &&
                          ((q.a_cl != 0 && q.cl_swap) || tma_ok(q.b, q.es, q.N, q.K, q.batch));
     if (q.a_cl != 0 && !use_tma) return kNotImplemented;
-    if (f32_tma_ok(*st, q)) return launch_f32(*st, q, stream);
+    if (q.b_lo != nullptr || f32_tma_ok(*st, q)) return launch_f32(*st, q, stream);  // (nothing else reads two parts)
     // A through tensor memory: every convolution and every other fp32 product (see contraction_ts.cuh)
     const int force_path = g_force_generic.load() & 0xff;
     if (force_path != 2 && !q.no_ts && !use_tma && (q.a.im2col || q.es == 4 || force_path == 3)) {
@@ -1488,7 +1498,8 @@ PadPlan pad_plan(const Problem& q) {
     };
     if (too_large(q.a, q.M) || too_large(q.b, q.N)) return PadPlan();
     if (a) plan.a_bytes = padded_line(q.a.k_major ? q.K : q.M, q.es) * static_cast<size_t>(q.a.k_major ? q.M : q.K);
-    if (b) plan.b_bytes = padded_line(q.b.k_major ? q.K : q.N, q.es) * static_cast<size_t>(q.b.k_major ? q.N : q.K);
+    // (fp32: two parts, which the loader warps that the copy spares round both)
+    if (b) plan.b_bytes = (q.es == 4 ? 2 : 1) * padded_line(q.b.k_major ? q.K : q.N, q.es) * static_cast<size_t>(q.b.k_major ? q.N : q.K);
     return plan;
 }
 
@@ -1512,6 +1523,10 @@ int pad_operands(Problem& q, const PadPlan& plan, char* ws, cudaStream_t stream)
     };
     if (plan.a) add(q.a, q.M, plan.a_bytes);
     if (plan.b) add(q.b, q.N, plan.b_bytes);
+    if (plan.b && q.es == 4) {
+        p.lo[n - 1] = static_cast<long long>(plan.b_bytes / 2);
+        q.b_lo = p.dst[n - 1] + p.lo[n - 1];
+    }
     clear_stale_error();
     const dim3 grid(static_cast<unsigned>(std::min<long long>((most + 255) / 256, 148 * 8)), static_cast<unsigned>(n));
     if (q.es == 2) pad_lines_kernel<2><<<grid, 256, 0, stream>>>(p);
@@ -1696,6 +1711,40 @@ int tri_args(int dtype, int& fmt, int& es, int layout, int& side, int& triangle,
         m = n;
         n = t;
     }
+    return kSuccess;
+}
+
+}  // namespace
+
+namespace {
+
+size_t split_bank_bytes(size_t num_kernels, size_t channels) { return 2 * num_kernels * channels * 4 + 256; }
+
+// The filter bank of an fp32 1x1 convolution (operand B of `q`, its lines contiguous and on 16-byte boundaries) as two
+// matrices of tf32 values at `ws`, for launches of several waves of tiles (see contraction_f32.cuh); with fewer tiles, or
+// without the room, the kernel rounds for itself. `dependent`: beside the kernel before it, whose end it waits for.
+int split_bank(Problem& q, const DeviceState& st, char* ws, const char* ws_end, bool dependent, cudaStream_t stream) {
+    q.b_round = true;
+    const size_t part = static_cast<size_t>(q.N) * static_cast<size_t>(q.K) * 4;
+    if (q.batch * ((q.M + kBM - 1) / kBM) * ((q.N + 127) / 128) <= st.num_sms || part / 16 >= (1ull << 31) || ws == nullptr ||
+        ws + 2 * part > ws_end)
+        return kSuccess;
+    PadLines p{};
+    p.src[0] = q.b.base;
+    p.dst[0] = ws;
+    p.src_pitch[0] = p.dst_pitch[0] = q.K * 4;
+    p.lines[0] = q.N;
+    p.length[0] = static_cast<int>(q.K);
+    p.lo[0] = static_cast<long long>(part);
+    p.wait = dependent ? 1 : 0;
+    clear_stale_error();
+    const unsigned grid = static_cast<unsigned>(std::min<size_t>((part / 16 + 255) / 256, 8ull * st.num_sms));
+    if (dependent) CUDA_TRY(launch_dependent(pad_lines_kernel<4>, grid, 256, 0, stream, p));
+    else pad_lines_kernel<4><<<grid, 256, 0, stream>>>(p);
+    g_launches.fetch_add(1);
+    CUDA_TRY(cudaGetLastError());
+    q.b.base = ws;
+    q.b_lo = ws + part;
     return kSuccess;
 }
 
@@ -2014,7 +2063,7 @@ size_t dlf_b200_conv2d_workspace_bytes(int dtype, size_t batches, size_t channel
     size_t need = (plain > row ? plain : row) + 256;
     // fp32 1x1 filters: the kept pixels with their channels contiguous
     if (es == 4 && group == 1 && kernel_h == 1 && kernel_w == 1) {
-        const size_t cl = batches * height * width * channels * 4 + 512;
+        const size_t cl = batches * height * width * channels * 4 + 512 + split_bank_bytes(num_kernels, channels);
         if (cl > need) need = cl;
     }
     // channels-last route (16-bit, one group): channels-last copy of the activations plus the
@@ -2127,7 +2176,15 @@ int dlf_b200_conv2d_fused(int dtype, size_t batches, size_t channels, size_t hei
             q.g.P = static_cast<int>(P);
             q.g.out_img_stride = static_cast<long long>(num_kernels) * P;
         }
-        return launch(q, static_cast<cudaStream_t>(stream));
+        DeviceState* st = nullptr;
+        int rc = ensure_device(&st);
+        if (rc != kSuccess) return rc;
+        if (q.es == 4 && f32_tma_ok(*st, q)) {
+            char* ws = workspace != nullptr ? align256(workspace) : nullptr;
+            rc = split_bank(q, *st, ws, static_cast<char*>(workspace) + workspace_bytes, false, static_cast<cudaStream_t>(stream));
+            if (rc != kSuccess) return rc;
+        }
+        return launch(q, static_cast<cudaStream_t>(stream), st);
     }
 
     // Other 1x1 filters without padding on fp32 data (a stride, or planes that are no 16-byte multiple): the kept
@@ -2170,6 +2227,9 @@ int dlf_b200_conv2d_fused(int dtype, size_t batches, size_t channels, size_t hei
             q.g.out_img_stride = static_cast<long long>(num_kernels) * P;
             q.pack_ws = nullptr;
             q.pack_ws_bytes = 0;
+            rc = split_bank(q, *st, align256(static_cast<char*>(workspace) + need), static_cast<char*>(workspace) + workspace_bytes, true,
+                            static_cast<cudaStream_t>(stream));
+            if (rc != kSuccess) return rc;
             return launch(q, static_cast<cudaStream_t>(stream), st);
         }
     }

@@ -173,6 +173,7 @@ struct Params {
                  // plain one-thread-per-output kernel (results stay valid), 0x4000 no programmatic
                  // dependent launch after the filter-packing grid (results stay valid)
     int dependent;  // the launch is a programmatic dependent of the kernel before it
+    int b_parts;    // contraction_f32_kernel: how operand B is split (F32_B_*)
 };
 
 struct PixelEntry {  // one output pixel of the current tile (implicit im2col operand)
@@ -287,6 +288,17 @@ __device__ __forceinline__ void split_tf32(uint32_t x, uint32_t& hi, uint32_t& l
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(xf));
     const float rest = xf - __uint_as_float(hi);
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(rest));
+}
+
+// The same for finite values, in integer arithmetic: lo is prepared for the truncation that it meets in the tensor core.
+// The addition carries the NaN that arithmetic returns, 0x7fffffff, past the exponent into -0; `check` turns NaN
+// when a rest is infinite or NaN, and the values it has seen have to be split by split_tf32 then.
+__device__ __forceinline__ void split_tf32_finite(uint32_t x, uint32_t& hi, uint32_t& lo, float& check) {
+    const float xf = __uint_as_float(x);
+    hi = (x + 0x1000u) & 0xffffe000u;
+    const float rest = xf - __uint_as_float(hi);
+    check = fmaf(0.0f, rest, check);
+    lo = __float_as_uint(rest) + 0x1000u;
 }
 
 __device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {

@@ -5,7 +5,13 @@
 // Every k-block of 32 k arrives raw, by TMA, in shared memory. Four splitter warps read their row
 // of A, split each value into tf32 hi (round to nearest) and lo, and put both into tensor memory;
 // two converter warps write lo = x - trunc(x) beside the raw tile of B, which the tensor core reads as the
-// tf32 truncation of itself. Three UMMAs per k-step accumulate lo*hi + hi*lo + hi*hi.
+// tf32 truncation of itself. Three UMMAs per k-step accumulate lo*hi + hi*lo + hi*hi. A value of B is then known to
+// 2^-21 of itself, one of A to 2^-23. Where this kernel stands in for one that rounds both parts of B too - the filters of
+// 1x1 convolutions, B operands off 16-byte boundaries - it does the same: with F32_B_ROUND the converters write hi over
+// the raw tile as well, with F32_B_SPLIT hi and lo are two matrices that a copy has written (pad_lines_kernel) and
+// TMA fetches both. Rounding in the kernel is for launches of one wave of tiles, which another launch would cost more
+// (64 -> 64 channels, 64 images of 8 x 8: 5.8 us truncated, 6.4 rounded here); over many waves the converters are too
+// slow for it (256 -> 256, 64 images of 56 x 56: 150 us truncated, 196 rounded here, 143 from two matrices).
 // The tensor core truncates when it adds into its accumulator, so it gets chunks of 8 k-blocks; eight
 // epilogue warps add the finished chunks with rounding to nearest, in registers (32 x 32*NB values per warp).
 //
@@ -29,6 +35,7 @@ namespace dlfb200 {
 constexpr int kF32Threads = 512;
 constexpr int kF32ChunkBlocks = 8;  // k-blocks per accumulator (256 k)
 constexpr int kF32MaxStages = 6;
+enum : int { F32_B_TRUNCATE = 0, F32_B_ROUND = 1, F32_B_SPLIT = 2 };  // Params::b_parts
 constexpr int f32_stage_bytes(int nb) { return kBM * 128 + 2 * 64 * nb * 128; }
 
 // Element offset of row i of D: i, or, for the rows of a convolution over the pixels of all images (out_nchw), the
@@ -61,13 +68,13 @@ __global__ void __launch_bounds__(256)
         if (p0 + row + i < P && c0 + lane < C) xp[(img * P + p0 + row + i) * C + c0 + lane] = tile[lane][row + i];
 }
 
-// A CTA has tiles of 128 x 64*NB, or, split > 1, the `split` CTAs of a cluster share one tile, each with its part of the k-blocks: for products with few tiles. The
-// partial tiles then meet in distributed shared memory (the operand ring, free by then, as [column][row]), where
-// CTA r adds up columns r*BN/split .. in rank order and writes them.
+// A CTA has tiles of 128 x 64*NB, or, split > 1, the `split` CTAs of a cluster share one tile, each with its part of the
+// k-blocks: for products with few tiles. The partial tiles then meet in distributed shared memory (the operand ring,
+// free by then, as [column][row]), where CTA r adds up columns r*BN/split .. in rank order and writes them.
 template <int NB>
 __global__ void __launch_bounds__(kF32Threads, 1)
     contraction_f32_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tmA,
-                           const __grid_constant__ CUtensorMap tmB, int split) {
+                           const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmBlo, int split) {
     constexpr int BN = 64 * NB;
     constexpr int BK = 32;
     constexpr uint32_t A_TILE = kBM * 128;
@@ -78,10 +85,10 @@ __global__ void __launch_bounds__(kF32Threads, 1)
     static_assert(A_COL0 + SLOTS * 64 <= 512, "two accumulators and the A slots share 512 columns");
 
     extern __shared__ uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t raw_full[kF32MaxStages];   // raw tiles of A and B landed (this CTA's)
+    __shared__ __align__(8) uint64_t raw_full[kF32MaxStages];   // tiles of A and B landed
     __shared__ __align__(8) uint64_t raw_empty[kF32MaxStages];  // splitters and UMMAs are done with the stage
-    __shared__ __align__(8) uint64_t conv_full[kF32MaxStages];  // lo image of B written (both CTAs')
-    __shared__ __align__(8) uint64_t slot_full[SLOTS];          // hi and lo of A in tensor memory (both CTAs')
+    __shared__ __align__(8) uint64_t conv_full[kF32MaxStages];  // lo image of B written
+    __shared__ __align__(8) uint64_t slot_full[SLOTS];          // hi and lo of A in tensor memory
     __shared__ __align__(8) uint64_t slot_empty[SLOTS];
     __shared__ __align__(8) uint64_t tfull_bar[2];
     __shared__ __align__(8) uint64_t tempty_bar[2];
@@ -124,6 +131,7 @@ __global__ void __launch_bounds__(kF32Threads, 1)
     if (warp == 12 && lane == 0) {
         ptx::tma_prefetch_desc(&tmA);
         ptx::tma_prefetch_desc(&tmB);
+        ptx::tma_prefetch_desc(&tmBlo);
     }
     ptx::tc_fence_before();
     __syncthreads();
@@ -241,20 +249,11 @@ __global__ void __launch_bounds__(kF32Threads, 1)
                     }
                 };
                 load_row(hi);
-                // hi = x rounded to tf32 (half away from zero), lo = the rest, prepared for the truncation it meets in
-                // the tensor core: split_tf32 in integer arithmetic, which the issue slots of these four warps have more
-                // room for (4096^3 624 us with the conversions, 582 so). It holds for finite values only - the addition
-                // carries the NaN that arithmetic returns, 0x7fffffff, past the exponent into -0 - and any other value
-                // leaves a rest that is not finite: such a row is split again by the conversions.
+                // (4096^3 624 us with the conversion instructions for every value, 582 so: these four warps have more
+                // issue slots for integer arithmetic)
                 float check = 0.0f;
 #pragma unroll
-                for (int k = 0; k < 32; ++k) {
-                    const float x = __uint_as_float(hi[k]);
-                    hi[k] = (hi[k] + 0x1000u) & 0xffffe000u;
-                    const float rest = x - __uint_as_float(hi[k]);
-                    check = fmaf(0.0f, rest, check);  // NaN if the rest is infinite or NaN
-                    lo[k] = __float_as_uint(rest) + 0x1000u;
-                }
+                for (int k = 0; k < 32; ++k) split_tf32_finite(hi[k], hi[k], lo[k], check);
                 if (check != 0.0f) {
                     load_row(hi);
 #pragma unroll
@@ -287,6 +286,7 @@ __global__ void __launch_bounds__(kF32Threads, 1)
     } else if (warp == 12) {
         // ------------------------------------------------------------ TMA producer
         const bool leader = ptx::elect_one();
+        const bool presplit = p.b_parts == F32_B_SPLIT;
         uint32_t s = 0, ph = 0;
         bool ok = true;
         for (int t = tile0; ok && t < p.total_tiles; t += gridDim.x) {
@@ -301,15 +301,19 @@ __global__ void __launch_bounds__(kF32Threads, 1)
                 const uint32_t bar = ptx::smem_u32(&raw_full[s]);
                 const uint32_t sA = smem0 + s * STAGE, sB = sA + A_TILE;
                 if (leader) {
-                    ptx::mbar_arrive_expect_tx(bar, A_TILE + B_TILE);
+                    ptx::mbar_arrive_expect_tx(bar, presplit ? A_TILE + 2 * B_TILE : A_TILE + B_TILE);
                     if (p.a.k_major) ptx::tma_load_3d(sA, &tmA, bar, (kb_begin + kb) * BK, m0, ba);
                     else ptx::tma_load_3d(sA, &tmA, bar, m0, (kb_begin + kb) * BK, ba);
-                    if (p.b.k_major) {
-                        ptx::tma_load_3d(sB, &tmB, bar, (kb_begin + kb) * BK, n0, bb);
-                    } else {
+                    for (int part_b = 0; part_b <= (presplit ? 1 : 0); ++part_b) {
+                        const uint32_t to = sB + part_b * B_TILE;
+                        const CUtensorMap* map = part_b ? &tmBlo : &tmB;
+                        if (p.b.k_major) {
+                            ptx::tma_load_3d(to, map, bar, (kb_begin + kb) * BK, n0, bb);
+                        } else {
 #pragma unroll
-                        for (int g = 0; g < BN / 32; ++g)
-                            ptx::tma_load_3d(sB + g * 4096, &tmB, bar, n0 + g * 32, (kb_begin + kb) * BK, bb);
+                            for (int g = 0; g < BN / 32; ++g)
+                                ptx::tma_load_3d(to + g * 4096, map, bar, n0 + g * 32, (kb_begin + kb) * BK, bb);
+                        }
                     }
                 }
                 __syncwarp();
@@ -326,6 +330,7 @@ __global__ void __launch_bounds__(kF32Threads, 1)
             const uint32_t b_step = (p.b.k_major ? 32u : 1024u) >> 4;
             const uint64_t db0 = ptx::make_smem_desc(smem0 + A_TILE, p.b.k_major ? 16u : BK * 128u, p.b.k_major ? 1024u : 512u,
                                                      p.b.k_major ? 2u : 1u);
+            const uint64_t* b_full = p.b_parts == F32_B_SPLIT ? raw_full : conv_full;
             uint32_t s = 0, ph = 0, slot = 0, sph = 0, buf = 0, tphase = 0;
             bool ok = true;
             for (int t = tile0; ok && t < p.total_tiles; t += gridDim.x) {
@@ -338,7 +343,7 @@ __global__ void __launch_bounds__(kF32Threads, 1)
                     const uint32_t d_tmem = tmem_base + buf * BN;
                     const int kb1 = min(kb0 + kF32ChunkBlocks, num_kb);
                     for (int kb = kb0; kb < kb1; ++kb) {
-                        if (!__all_sync(0xffffffffu, ptx::mbar_wait_bounded(ptx::smem_u32(&conv_full[s]), ph, abort_p, wait_limit) &&
+                        if (!__all_sync(0xffffffffu, ptx::mbar_wait_bounded(ptx::smem_u32(&b_full[s]), ph, abort_p, wait_limit) &&
                                                          ptx::mbar_wait_bounded(ptx::smem_u32(&slot_full[slot]), sph, abort_p, wait_limit))) {
                             ok = false;
                             break;
@@ -376,7 +381,7 @@ __global__ void __launch_bounds__(kF32Threads, 1)
                 }
             }
         }
-    } else {
+    } else if (p.b_parts != F32_B_SPLIT) {
         // ------------------------------------------------------------ converters: lo image of B
         const uint32_t ct = threadIdx.x - 14 * 32;  // 0..63
         uint32_t s = 0, ph = 0;
@@ -388,15 +393,49 @@ __global__ void __launch_bounds__(kF32Threads, 1)
                     break;
                 }
                 const uint32_t sB = smem0 + s * STAGE + A_TILE + ct * 16u;
+                if (p.b_parts == F32_B_ROUND) {
+                    // four chunks at a time: one branch on their finiteness, and as many loads in flight
+#pragma unroll 2
+                    for (uint32_t o = 0; o < B_TILE; o += 4u * 64u * 16u) {
+                        uint32_t hi[16], lo[16];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const uint4 v = ld_shared_v4(sB + o + i * 1024u);
+                            hi[4 * i] = v.x;
+                            hi[4 * i + 1] = v.y;
+                            hi[4 * i + 2] = v.z;
+                            hi[4 * i + 3] = v.w;
+                        }
+                        float check = 0.0f;
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) split_tf32_finite(hi[i], hi[i], lo[i], check);
+                        if (check != 0.0f) {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                const uint4 v = ld_shared_v4(sB + o + i * 1024u);
+                                split_tf32(v.x, hi[4 * i], lo[4 * i]);
+                                split_tf32(v.y, hi[4 * i + 1], lo[4 * i + 1]);
+                                split_tf32(v.z, hi[4 * i + 2], lo[4 * i + 2]);
+                                split_tf32(v.w, hi[4 * i + 3], lo[4 * i + 3]);
+                            }
+                        }
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            st_shared_v4(sB + o + i * 1024u, make_uint4(hi[4 * i], hi[4 * i + 1], hi[4 * i + 2], hi[4 * i + 3]));
+                            st_shared_v4(sB + B_TILE + o + i * 1024u, make_uint4(lo[4 * i], lo[4 * i + 1], lo[4 * i + 2], lo[4 * i + 3]));
+                        }
+                    }
+                } else {
 #pragma unroll 4
-                for (uint32_t o = 0; o < B_TILE; o += 64u * 16u) {
-                    const uint4 v = ld_shared_v4(sB + o);
-                    uint4 lo;
-                    lo.x = __float_as_uint(__uint_as_float(v.x) - __uint_as_float(v.x & 0xffffe000u));
-                    lo.y = __float_as_uint(__uint_as_float(v.y) - __uint_as_float(v.y & 0xffffe000u));
-                    lo.z = __float_as_uint(__uint_as_float(v.z) - __uint_as_float(v.z & 0xffffe000u));
-                    lo.w = __float_as_uint(__uint_as_float(v.w) - __uint_as_float(v.w & 0xffffe000u));
-                    st_shared_v4(sB + B_TILE + o, lo);
+                    for (uint32_t o = 0; o < B_TILE; o += 64u * 16u) {
+                        const uint4 v = ld_shared_v4(sB + o);
+                        uint4 lo;
+                        lo.x = __float_as_uint(__uint_as_float(v.x) - __uint_as_float(v.x & 0xffffe000u));
+                        lo.y = __float_as_uint(__uint_as_float(v.y) - __uint_as_float(v.y & 0xffffe000u));
+                        lo.z = __float_as_uint(__uint_as_float(v.z) - __uint_as_float(v.z & 0xffffe000u));
+                        lo.w = __float_as_uint(__uint_as_float(v.w) - __uint_as_float(v.w & 0xffffe000u));
+                        st_shared_v4(sB + B_TILE + o, lo);
+                    }
                 }
                 ptx::fence_proxy_async_smem();
                 __syncwarp();

@@ -13,6 +13,7 @@
 
 #include <cstdint>
 
+#include "contraction.cuh"
 #include "ptx.cuh"
 
 namespace dlfb200 {
@@ -95,6 +96,8 @@ __global__ void splitk_reduce_kernel(T* __restrict__ d, long long ldd, const flo
 // Copies of matrices whose lines start anywhere (an odd leading dimension or offset) with lines on 16-byte
 // boundaries, the form the tensor maps take: up to two matrices per launch (blockIdx.y). A thread writes
 // one 16-byte chunk; the elements past a line's end are zero. HBM-bound (each matrix read and written once).
+// fp32 lines can be written as the two tf32 parts that contraction_f32_kernel reads (operand B; F32_B_SPLIT: 2001 x 2003 x
+// 2005 118 us, 110 with one part that the kernel truncates, 208 by the loader warps, which round both as this does).
 // 16-bit lines that start on an odd element are read as aligned 32-bit words and shifted together.
 // bf16 1111 x 1537 x 777 with both operands odd: 6 us for the copies, the product 62 -> 11 us.
 struct PadLines {
@@ -103,6 +106,8 @@ struct PadLines {
     long long src_pitch[2], dst_pitch[2];  // bytes
     long long lines[2];
     int length[2];                         // elements of a line
+    long long lo[2];                       // fp32: != 0: tf32 hi goes to dst and the rest, as tf32, this many bytes behind it
+    int wait;                              // the launch is a programmatic dependent: it ends after the kernel before it
 };
 template <int ES>
 __global__ void __launch_bounds__(256) pad_lines_kernel(const PadLines p) {
@@ -141,8 +146,18 @@ __global__ void __launch_bounds__(256) pad_lines_kernel(const PadLines p) {
             }
             v = make_uint4(e[0], e[1], e[2], e[3]);
         }
-        *reinterpret_cast<uint4*>(p.dst[m] + line * p.dst_pitch[m] + static_cast<long long>(e0) * ES) = v;
+        char* dst = p.dst[m] + line * p.dst_pitch[m] + static_cast<long long>(e0) * ES;
+        if (ES == 4 && p.lo[m] != 0) {
+            uint4 lo;
+            split_tf32(v.x, v.x, lo.x);
+            split_tf32(v.y, v.y, lo.y);
+            split_tf32(v.z, v.z, lo.z);
+            split_tf32(v.w, v.w, lo.w);
+            *reinterpret_cast<uint4*>(dst + p.lo[m]) = lo;
+        }
+        *reinterpret_cast<uint4*>(dst) = v;
     }
+    if (p.wait) ptx::wait_for_dependencies();
 }
 
 constexpr int kTrsmOrder = 1024;   // unknowns one launch solves; longer systems are cut into blocks of this order

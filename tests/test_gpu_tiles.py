@@ -298,3 +298,39 @@ def test_a_captured_unaligned_product_survives_larger_ones(lib):
     graph.replay()
     assert float((y - a @ b).norm() / y.norm()) <= 2e-3  # (torch's product of fp32 matrices may use tf32)
     assert all(bool((o == 7).all()) for o in others)
+
+
+@pytest.mark.parametrize("size,stride", [(8, 1), (7, 1), (14, 2)], ids=["planes of 16 bytes", "odd planes", "stride 2"])
+@pytest.mark.parametrize("channels,filters", [(48, 64), (48, 200)])
+def test_pointwise_fp32_filters_keep_all_but_the_last_bit(lib, channels, filters, size, stride):
+    """A 1x1 filter bank over pixels that are one in one channel each: what comes out are the weights as the kernel
+    holds them. Rounded to tf32 (11 bits), the rest rounded to tf32 again: within 2^-23 of the value."""
+    from dlf_b200 import gdnn
+    rng = np.random.default_rng(filters)
+    f = gdnn.Filter2D((1, channels, size, size), (filters, channels, 1, 1)).strides(stride, stride)
+    pixels = f.output_h * f.output_w
+    assert pixels >= channels
+    X = np.zeros((channels, size, size), np.float32)
+    kept = X[:, ::stride, ::stride]
+    for c in range(channels):
+        kept[c, c // f.output_w, c % f.output_w] = 1.0
+    W = rng.normal(size=(filters, channels)).astype(np.float32)
+    Y = torch.empty(f.output_shape(), device="cuda")
+    gdnn.conv2d_filter(torch.from_numpy(X).cuda(), torch.from_numpy(W).cuda(), Y, f)
+    got = Y.cpu().numpy().reshape(filters, pixels)[:, :channels]
+    assert (np.abs(got.astype(np.float64) - W) <= 2.0 ** -23 * np.abs(W)).all()
+
+
+@pytest.mark.parametrize("ta,tb", [(False, False), (True, False), (False, True), (True, True)])
+def test_copied_fp32_operands_keep_all_but_the_last_bit(lib, ta, tb):
+    """Operands off 16-byte boundaries times the identity: within 2^-23 of the value, on either side."""
+    from dlf_b200 import tensor
+    rng = np.random.default_rng(3)
+    n = 261
+    for first in (True, False):
+        M = torch.from_numpy(rng.normal(size=(n, n)).astype(np.float32)).cuda()
+        I = torch.eye(n, device="cuda")
+        A, B = (M, I) if first else (I, M)
+        got = tensor.matmul(A.t() if ta else A, B.t() if tb else B, torch.empty(n, n, device="cuda"))
+        want = M.t() if (ta if first else tb) else M
+        assert bool(((got.double() - want.double()).abs() <= 2.0 ** -23 * want.double().abs()).all())
