@@ -290,15 +290,16 @@ __device__ __forceinline__ void split_tf32(uint32_t x, uint32_t& hi, uint32_t& l
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(rest));
 }
 
-// The same for finite values, in integer arithmetic: lo is prepared for the truncation that it meets in the tensor core.
-// The addition carries the NaN that arithmetic returns, 0x7fffffff, past the exponent into -0; `check` turns NaN
-// when a rest is infinite or NaN, and the values it has seen have to be split by split_tf32 then.
-__device__ __forceinline__ void split_tf32_finite(uint32_t x, uint32_t& hi, uint32_t& lo, float& check) {
-    const float xf = __uint_as_float(x);
-    hi = (x + 0x1000u) & 0xffffe000u;
-    const float rest = xf - __uint_as_float(hi);
-    check = fmaf(0.0f, rest, check);
-    lo = __float_as_uint(rest) + 0x1000u;
+// The same values for what reads tf32 by truncation, without the conversion instructions. rest = x - hi is a whole number of
+// units in the last place of x, 4096 at most; rest + rest / 2048 lies less than a unit of 11 bits above it and, where the
+// twelfth bit is one, above the middle: truncated, it is rest rounded half away from zero. Both operations keep a
+// NaN, and the rest of a NaN or of an infinity is one, whatever became of hi (the integer addition carries the NaN that
+// arithmetic returns, 0x7fffffff, past the exponent into -0).
+__device__ __forceinline__ void split_tf32_int(uint32_t x, uint32_t& hi, uint32_t& lo) {
+    const uint32_t rounded = (x + 0x1000u) & 0xffffe000u;
+    const float rest = __uint_as_float(x) - __uint_as_float(rounded);
+    hi = rounded;
+    lo = __float_as_uint(fmaf(rest, 1.0f / 2048.0f, rest));
 }
 
 __device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {

@@ -232,33 +232,23 @@ __global__ void __launch_bounds__(kF32Threads, 1)
                 }
                 const uint32_t sA = smem0 + s * STAGE;
                 uint32_t hi[32], lo[32];
-                auto load_row = [&](uint32_t (&x)[32]) {
-                    if (p.a.k_major) {
+                if (p.a.k_major) {
 #pragma unroll
-                        for (int c = 0; c < 8; ++c) {
-                            const uint4 u = ld_shared_v4(sA + L * 128u + ((c ^ (L & 7)) << 4));
-                            x[4 * c + 0] = u.x;
-                            x[4 * c + 1] = u.y;
-                            x[4 * c + 2] = u.z;
-                            x[4 * c + 3] = u.w;
-                        }
-                    } else {
-#pragma unroll
-                        for (int k = 0; k < 32; ++k)
-                            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(x[k]) : "r"(sA + k * (kBM * 4) + L * 4) : "memory");
+                    for (int c = 0; c < 8; ++c) {
+                        const uint4 u = ld_shared_v4(sA + L * 128u + ((c ^ (L & 7)) << 4));
+                        hi[4 * c + 0] = u.x;
+                        hi[4 * c + 1] = u.y;
+                        hi[4 * c + 2] = u.z;
+                        hi[4 * c + 3] = u.w;
                     }
-                };
-                load_row(hi);
-                // (4096^3 624 us with the conversion instructions for every value, 582 so: these four warps have more
-                // issue slots for integer arithmetic)
-                float check = 0.0f;
+                } else {
 #pragma unroll
-                for (int k = 0; k < 32; ++k) split_tf32_finite(hi[k], hi[k], lo[k], check);
-                if (check != 0.0f) {
-                    load_row(hi);
-#pragma unroll
-                    for (int k = 0; k < 32; ++k) split_tf32(hi[k], hi[k], lo[k]);
+                    for (int k = 0; k < 32; ++k)
+                        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(hi[k]) : "r"(sA + k * (kBM * 4) + L * 4) : "memory");
                 }
+                // (4096^3 7 % slower with the conversion instructions of split_tf32)
+#pragma unroll
+                for (int k = 0; k < 32; ++k) split_tf32_int(hi[k], hi[k], lo[k]);
                 __syncwarp();
                 if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&raw_empty[s]));
                 if (!__all_sync(0xffffffffu, ptx::mbar_wait_bounded(ptx::smem_u32(&slot_empty[slot]), sph ^ 1u, abort_p, wait_limit))) {
@@ -394,36 +384,16 @@ __global__ void __launch_bounds__(kF32Threads, 1)
                 }
                 const uint32_t sB = smem0 + s * STAGE + A_TILE + ct * 16u;
                 if (p.b_parts == F32_B_ROUND) {
-                    // four chunks at a time: one branch on their finiteness, and as many loads in flight
-#pragma unroll 2
-                    for (uint32_t o = 0; o < B_TILE; o += 4u * 64u * 16u) {
-                        uint32_t hi[16], lo[16];
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const uint4 v = ld_shared_v4(sB + o + i * 1024u);
-                            hi[4 * i] = v.x;
-                            hi[4 * i + 1] = v.y;
-                            hi[4 * i + 2] = v.z;
-                            hi[4 * i + 3] = v.w;
-                        }
-                        float check = 0.0f;
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) split_tf32_finite(hi[i], hi[i], lo[i], check);
-                        if (check != 0.0f) {
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                const uint4 v = ld_shared_v4(sB + o + i * 1024u);
-                                split_tf32(v.x, hi[4 * i], lo[4 * i]);
-                                split_tf32(v.y, hi[4 * i + 1], lo[4 * i + 1]);
-                                split_tf32(v.z, hi[4 * i + 2], lo[4 * i + 2]);
-                                split_tf32(v.w, hi[4 * i + 3], lo[4 * i + 3]);
-                            }
-                        }
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            st_shared_v4(sB + o + i * 1024u, make_uint4(hi[4 * i], hi[4 * i + 1], hi[4 * i + 2], hi[4 * i + 3]));
-                            st_shared_v4(sB + B_TILE + o + i * 1024u, make_uint4(lo[4 * i], lo[4 * i + 1], lo[4 * i + 2], lo[4 * i + 3]));
-                        }
+#pragma unroll 4
+                    for (uint32_t o = 0; o < B_TILE; o += 64u * 16u) {
+                        const uint4 v = ld_shared_v4(sB + o);
+                        uint4 hi, lo;
+                        split_tf32_int(v.x, hi.x, lo.x);
+                        split_tf32_int(v.y, hi.y, lo.y);
+                        split_tf32_int(v.z, hi.z, lo.z);
+                        split_tf32_int(v.w, hi.w, lo.w);
+                        st_shared_v4(sB + o, hi);
+                        st_shared_v4(sB + B_TILE + o, lo);
                     }
                 } else {
 #pragma unroll 4

@@ -148,11 +148,12 @@ __global__ void __launch_bounds__(256) pad_lines_kernel(const PadLines p) {
         }
         char* dst = p.dst[m] + line * p.dst_pitch[m] + static_cast<long long>(e0) * ES;
         if (ES == 4 && p.lo[m] != 0) {
+            const uint4 x = v;
             uint4 lo;
-            split_tf32(v.x, v.x, lo.x);
-            split_tf32(v.y, v.y, lo.y);
-            split_tf32(v.z, v.z, lo.z);
-            split_tf32(v.w, v.w, lo.w);
+            split_tf32_int(x.x, v.x, lo.x);
+            split_tf32_int(x.y, v.y, lo.y);
+            split_tf32_int(x.z, v.z, lo.z);
+            split_tf32_int(x.w, v.w, lo.w);
             *reinterpret_cast<uint4*>(dst + p.lo[m]) = lo;
         }
         *reinterpret_cast<uint4*>(dst) = v;
