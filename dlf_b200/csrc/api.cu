@@ -53,6 +53,7 @@ enum : int {
 
 constexpr int kMaxDevices = 64;
 constexpr int kSmemPerBlockOptin = 232448;  // 227 KB
+constexpr int kB200Sms = 148;  // for sizes that are asked for without a device at hand
 
 struct DeviceState {
     bool ready = false;
@@ -378,6 +379,7 @@ struct Problem {
     bool d_f32 = false;  // 16-bit operands with fp32 output (partial products of a K-split GEMM)
     bool b_round = false;  // contraction_f32_kernel: both parts of operand B rounded (F32_B_ROUND)
     const char* b_lo = nullptr;  // operand B as two matrices of tf32 values, laid out alike: b.base and this (F32_B_SPLIT)
+    bool short_chunks = false;   // contraction_ts_kernel, fp32: sums of 8 k-blocks from K > 256 on, not only from K > 512
     bool no_ts = false;  // convolution whose taps overflow the k table's 16/32-bit fields
 };
 
@@ -639,7 +641,7 @@ int launch_ts(const DeviceState& st, const Problem& q, cudaStream_t stream) {
     // float[BN][128] sum array (96 KB at 192 columns) and two operand stages of 48 KB limit such
     // tiles to 192 columns, which is also the widest tile that leaves room for two accumulators.
     const long long num_kb_all = (q.K + BK - 1) / BK;
-    const int kc_blocks = (q.es == 4 && num_kb_all > 16 && !(g_force_generic.load() & 0x1000)) ? 8 : 0;
+    const int kc_blocks = (q.es == 4 && num_kb_all > (q.short_chunks ? 8 : 16) && !(g_force_generic.load() & 0x1000)) ? 8 : 0;
     int bn = choose_bn_ts(q, st.num_sms, kc_blocks ? 192 : 256, a_cols, num_kb_all);
     const int forced = g_force_bn.load() & 0xffff;
     if (forced >= 64 && forced <= (kc_blocks ? 192 : 256) && forced % 32 == 0) bn = forced;
@@ -1475,6 +1477,7 @@ namespace {
 
 struct PadPlan {
     bool a = false, b = false;
+    bool b_split = false;  // fp32: the copy of B is two matrices of tf32 values; else the kernel rounds both parts (contraction_f32.cuh)
     size_t a_bytes = 0, b_bytes = 0;
     size_t bytes() const { return a_bytes + b_bytes; }
 };
@@ -1489,7 +1492,7 @@ PadPlan pad_plan(const Problem& q) {
     // (bf16 1111 x 1537 x 777, 13 blocks: 62 us by the loader warps, 6 + 11 us with the copy; fp32 60 x 72 x 50,
     // two blocks: 11.5 us by the loader warps, and the copy's launch alone takes 3)
     const long long tiles = ((q.M + kBM - 1) / kBM) * ((q.N + 127) / 128);
-    const long long walk = (tiles + 147) / 148 * ((q.K * q.es + 127) / 128);
+    const long long walk = (tiles + kB200Sms - 1) / kB200Sms * ((q.K * q.es + 127) / 128);
     if (walk < 4) return plan;
     plan.a = a;
     plan.b = b;
@@ -1498,8 +1501,8 @@ PadPlan pad_plan(const Problem& q) {
     };
     if (too_large(q.a, q.M) || too_large(q.b, q.N)) return PadPlan();
     if (a) plan.a_bytes = padded_line(q.a.k_major ? q.K : q.M, q.es) * static_cast<size_t>(q.a.k_major ? q.M : q.K);
-    // (fp32: two parts, which the loader warps that the copy spares round both)
-    if (b) plan.b_bytes = (q.es == 4 ? 2 : 1) * padded_line(q.b.k_major ? q.K : q.N, q.es) * static_cast<size_t>(q.b.k_major ? q.N : q.K);
+    plan.b_split = b && q.es == 4 && tiles > kB200Sms;
+    if (b) plan.b_bytes = (plan.b_split ? 2 : 1) * padded_line(q.b.k_major ? q.K : q.N, q.es) * static_cast<size_t>(q.b.k_major ? q.N : q.K);
     return plan;
 }
 
@@ -1523,7 +1526,8 @@ int pad_operands(Problem& q, const PadPlan& plan, char* ws, cudaStream_t stream)
     };
     if (plan.a) add(q.a, q.M, plan.a_bytes);
     if (plan.b) add(q.b, q.N, plan.b_bytes);
-    if (plan.b && q.es == 4) {
+    q.b_round = plan.b;
+    if (plan.b_split) {
         p.lo[n - 1] = static_cast<long long>(plan.b_bytes / 2);
         q.b_lo = p.dst[n - 1] + p.lo[n - 1];
     }
@@ -1718,15 +1722,42 @@ int tri_args(int dtype, int& fmt, int& es, int layout, int& side, int& triangle,
 
 namespace {
 
+// What serves a 1x1 fp32 convolution without padding whose operands contraction_f32_kernel can be given:
+//   PW_BATCHED  a product per image on the planes as they are (stride 1, planes of whole 16 bytes),
+//   PW_COPY     one product over the pixels of all images, copied with their channels contiguous,
+//   PW_GATHER   contraction_ts_kernel, which gathers.
+// The lines are where measured times crossed (267 shapes of 1-256 images, 4-2048 channels, planes of 2 x 2 to 56 x 56; within
+// 1 % of the best of the three on average, and of 19 % at worst). A product per image fills its 128-row tiles with one
+// image's pixels, which pays when three quarters of the rows are in use (512 -> 512, 256 images: 4 x 4 gather 26, per
+// image 85 us; 10 x 10 97 and 88) or all tiles run at once anyway (256 -> 256, 32 images of 8 x 8: 15.1 and 11.6). With fewer
+// than 8 channels and few filters there is nothing but output to write, and the gathering kernel writes it faster (4 -> 24,
+// 219 images of 8 x 61: 20.6 and 29.4). The copy pays when it leaves few tiles, which clusters share (64 images 1024 -> 256
+// 4 x 4: gather 32.8, copied 18.0 us), or is small against the output (105 images 4 -> 377 28 x 28: 109 and 76); else its
+// traffic costs more than the gather (176 -> 181, 155 images 26 x 8, stride 2: 18.0 and 18.8; 32 -> 13: 8.8 and 8.9).
+enum { PW_GATHER, PW_BATCHED, PW_COPY };
+
+int pointwise_route(int num_sms, size_t batches, size_t channels, size_t pixels, size_t num_kernels, bool planes_aligned) {
+    const size_t row_tiles = batches * ((pixels + kBM - 1) / kBM), col_tiles = (num_kernels + 127) / 128;
+    if (planes_aligned) {
+        if (channels < 8 && num_kernels <= 64 && row_tiles > static_cast<size_t>(num_sms)) return PW_GATHER;
+        if (4 * batches * pixels >= 3 * kBM * row_tiles || 10 * row_tiles * col_tiles <= 7 * static_cast<size_t>(num_sms)) return PW_BATCHED;
+    }
+    const size_t copied_tiles = (batches * pixels + kBM - 1) / kBM * col_tiles;
+    return 2 * copied_tiles <= static_cast<size_t>(num_sms) || 2 * num_kernels >= 3 * channels ? PW_COPY : PW_GATHER;
+}
+
 size_t split_bank_bytes(size_t num_kernels, size_t channels) { return 2 * num_kernels * channels * 4 + 256; }
 
 // The filter bank of an fp32 1x1 convolution (operand B of `q`, its lines contiguous and on 16-byte boundaries) as two
-// matrices of tf32 values at `ws`, for launches of several waves of tiles (see contraction_f32.cuh); with fewer tiles, or
-// without the room, the kernel rounds for itself. `dependent`: beside the kernel before it, whose end it waits for.
+// matrices of tf32 values at `ws`. That launch takes 2 to 3 us, rounding in the kernel some 300 clocks a k-block (see
+// contraction_f32.cuh): it pays from a dozen k-blocks one after the other (8 images of 64 x 64, 12 -> 8: one k-block in two
+// waves of tiles, 8.6 us and 11.7 with the launch). Else, or without the room, the kernel rounds for itself.
+// `dependent`: beside the kernel before it, whose end it waits for.
 int split_bank(Problem& q, const DeviceState& st, char* ws, const char* ws_end, bool dependent, cudaStream_t stream) {
     q.b_round = true;
     const size_t part = static_cast<size_t>(q.N) * static_cast<size_t>(q.K) * 4;
-    if (q.batch * ((q.M + kBM - 1) / kBM) * ((q.N + 127) / 128) <= st.num_sms || part / 16 >= (1ull << 31) || ws == nullptr ||
+    const long long tiles = q.batch * ((q.M + kBM - 1) / kBM) * ((q.N + 127) / 128);
+    if (tiles <= st.num_sms || (tiles + st.num_sms - 1) / st.num_sms * ((q.K + 31) / 32) <= 12 || part / 16 >= (1ull << 31) || ws == nullptr ||
         ws + 2 * part > ws_end)
         return kSuccess;
     PadLines p{};
@@ -2045,7 +2076,7 @@ int dlf_b200_gemm_batched_noalloc(int dtype, int layout, int trans_a, int trans_
 }
 
 size_t dlf_b200_conv2d_workspace_bytes(int dtype, size_t batches, size_t channels, size_t height, size_t width,
-                                       size_t, size_t, size_t num_kernels, size_t group, size_t kernel_h,
+                                       size_t output_h, size_t output_w, size_t num_kernels, size_t group, size_t kernel_h,
                                        size_t kernel_w) {
     // Optional scratch: the filter bank re-laid as the kernel's shared-memory stage images (a few
     // hundred KB to a few MB). The im2col matrix itself is never materialised. An upper bound over
@@ -2061,9 +2092,12 @@ size_t dlf_b200_conv2d_workspace_bytes(int dtype, size_t batches, size_t channel
     const size_t row = group * ((ng + 255) / 256 * 256 + 256) * 128 * dup *
                        ((cg * kernel_h * (kernel_w + 8) + bk - 1) / bk + 8);
     size_t need = (plain > row ? plain : row) + 256;
-    // fp32 1x1 filters: the kept pixels with their channels contiguous
-    if (es == 4 && group == 1 && kernel_h == 1 && kernel_w == 1) {
-        const size_t cl = batches * height * width * channels * 4 + 512 + split_bank_bytes(num_kernels, channels);
+    // fp32 1x1 filters where they are copied: the kept pixels with their channels contiguous, and the split filters
+    if (es == 4 && group == 1 && kernel_h == 1 && kernel_w == 1 && channels % 4 == 0 && output_h <= height && output_w <= width) {
+        const size_t pixels = output_h * output_w;
+        const bool aligned = output_h == height && output_w == width && pixels % 4 == 0;
+        size_t cl = split_bank_bytes(num_kernels, channels) + 256;
+        if (pointwise_route(kB200Sms, batches, channels, pixels, num_kernels, aligned) == PW_COPY) cl += batches * pixels * channels * 4 + 256;
         if (cl > need) need = cl;
     }
     // channels-last route (16-bit, one group): channels-last copy of the activations plus the
@@ -2130,13 +2164,35 @@ int dlf_b200_conv2d_fused(int dtype, size_t batches, size_t channels, size_t hei
     StreamDevice sd(static_cast<cudaStream_t>(stream));
     if (sd.rc != kSuccess) return sd.rc;
 
+    // fp32 1x1 filters without padding: which kernel (see pointwise_route), and where the copied pixels go
+    const bool pointwise = q.es == 4 && group == 1 && kernel_h == 1 && kernel_w == 1 && pad_top == 0 && pad_left == 0 && channels % 4 == 0 &&
+                           (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && (output_h - 1) * stride_h < height && (output_w - 1) * stride_w < width &&
+                           g_force_generic.load() == 0 && g_force_bn.load() == 0 && P <= INT_MAX / 2 && channels < INT_MAX - 512 && num_kernels < INT_MAX - 512;
+    int route = PW_GATHER;
+    char* const pixel_ws = workspace != nullptr ? align256(workspace) : nullptr;
+    const char* const ws_end = static_cast<const char*>(workspace) + workspace_bytes;
+    const size_t pixel_bytes = batches * static_cast<size_t>(P) * channels * 4;
+    if (pointwise) {
+        DeviceState* st = nullptr;
+        const int rc = ensure_device(&st);
+        if (rc != kSuccess) return rc;
+        const bool aligned = stride_h == 1 && stride_w == 1 && output_h == height && output_w == width && P % 4 == 0 &&
+                             (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+        if (st->static_smem_f32 >= 0) route = pointwise_route(st->num_sms, batches, channels, static_cast<size_t>(P), num_kernels, aligned);
+        const bool countable = static_cast<long long>(batches) * P < INT_MAX - 512;  // (pixels of all images as the rows of one problem)
+        if (route == PW_COPY && (pixel_ws == nullptr || pixel_ws + pixel_bytes > ws_end || batches >= 65536 || (channels + 31) / 32 >= 65536))
+            route = aligned ? PW_BATCHED : PW_GATHER;
+        if (!countable) route = aligned ? PW_BATCHED : PW_GATHER;
+        q.short_chunks = true;  // (gathered: in chunks of the same length as the products)
+    }
+
     // A 1x1, stride-1, unpadded convolution is a batched GEMM over the images,
     //     Y[b] (Cout x P) = W (Cout x Cin) * X[b] (Cin x P),
     // exactly the reference's convWithIm2Col shortcut (gpgpu/src/gdnn.cpp:1512-1559: weights
     // shared with stride 0). With TMA-compatible strides it takes the TMA-fed kernel.
     if (kernel_h == 1 && kernel_w == 1 && stride_h == 1 && stride_w == 1 && pad_top == 0 &&
         pad_left == 0 && output_h == height && output_w == width && group == 1 &&
-        (q.es == 2 || (g_force_generic.load() == 0 && g_force_bn.load() == 0 && P <= INT_MAX / 2)) &&
+        (q.es == 2 || route == PW_BATCHED) &&
         (P * q.es) % 16 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 &&
         (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && (channels * q.es) % 16 == 0 &&
         !(g_force_generic.load() & 0xff)) {
@@ -2180,58 +2236,48 @@ int dlf_b200_conv2d_fused(int dtype, size_t batches, size_t channels, size_t hei
         int rc = ensure_device(&st);
         if (rc != kSuccess) return rc;
         if (q.es == 4 && f32_tma_ok(*st, q)) {
-            char* ws = workspace != nullptr ? align256(workspace) : nullptr;
-            rc = split_bank(q, *st, ws, static_cast<char*>(workspace) + workspace_bytes, false, static_cast<cudaStream_t>(stream));
+            rc = split_bank(q, *st, pixel_ws, ws_end, false, static_cast<cudaStream_t>(stream));
             if (rc != kSuccess) return rc;
         }
         return launch(q, static_cast<cudaStream_t>(stream), st);
     }
 
-    // Other 1x1 filters without padding on fp32 data (a stride, or planes that are no 16-byte multiple): the kept
-    // pixels are copied with their channels contiguous, after which the layer is one product over all images,
+    // The kept pixels are copied with their channels contiguous, after which the layer is one product over all images,
     // written to NCHW by lanes that hold pixels. (ResNet-50 at batch 8 has eleven such layers: 30 us each by the
     // gathering kernel; the whole forward 1416 -> 1274 us.)
-    if (q.es == 4 && group == 1 && kernel_h == 1 && kernel_w == 1 && pad_top == 0 && pad_left == 0 && channels % 4 == 0 &&
-        (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && (output_h - 1) * stride_h < height && (output_w - 1) * stride_w < width &&
-        workspace != nullptr && g_force_generic.load() == 0 && g_force_bn.load() == 0 && batches < 65536 &&
-        static_cast<long long>(batches) * P < INT_MAX - 512 && (channels + 31) / 32 < 65536 && channels < INT_MAX - 512 &&
-        num_kernels < INT_MAX - 512 && static_cast<long long>(height) * width < INT_MAX) {
-        char* xp = align256(workspace);
-        const size_t need = static_cast<size_t>(xp - static_cast<char*>(workspace)) + batches * static_cast<size_t>(P) * channels * 4;
+    if (route == PW_COPY) {
         DeviceState* st = nullptr;
         int rc = ensure_device(&st);
         if (rc != kSuccess) return rc;
-        if (workspace_bytes >= need && st->static_smem_f32 >= 0) {
-            clear_stale_error();
-            const dim3 grid(static_cast<unsigned>((P + 31) / 32), static_cast<unsigned>((channels + 31) / 32), static_cast<unsigned>(batches));
-            f32_pack_pixels_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-                static_cast<const float*>(x), reinterpret_cast<float*>(xp), static_cast<int>(channels),
-                static_cast<long long>(height) * width, static_cast<int>(width), static_cast<int>(P), static_cast<int>(output_w),
-                static_cast<int>(stride_h), static_cast<int>(stride_w));
-            g_launches.fetch_add(1);
-            CUDA_TRY(cudaGetLastError());
-            q.M = static_cast<long long>(batches) * P;
-            q.N = static_cast<long long>(num_kernels);
-            q.K = static_cast<long long>(channels);
-            q.a.base = xp;
-            q.a.k_major = 1;
-            q.a.ld = static_cast<long long>(channels);
-            q.b.base = static_cast<const char*>(w);
-            q.b.k_major = 1;
-            q.b.ld = static_cast<long long>(channels);
-            q.d = static_cast<char*>(y);
-            q.ldd = P;
-            q.bias = static_cast<const char*>(bias);
-            q.out_nchw = 1;
-            q.g.P = static_cast<int>(P);
-            q.g.out_img_stride = static_cast<long long>(num_kernels) * P;
-            q.pack_ws = nullptr;
-            q.pack_ws_bytes = 0;
-            rc = split_bank(q, *st, align256(static_cast<char*>(workspace) + need), static_cast<char*>(workspace) + workspace_bytes, true,
-                            static_cast<cudaStream_t>(stream));
-            if (rc != kSuccess) return rc;
-            return launch(q, static_cast<cudaStream_t>(stream), st);
-        }
+        clear_stale_error();
+        const dim3 grid(static_cast<unsigned>((P + 31) / 32), static_cast<unsigned>((channels + 31) / 32), static_cast<unsigned>(batches));
+        f32_pack_pixels_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+            static_cast<const float*>(x), reinterpret_cast<float*>(pixel_ws), static_cast<int>(channels),
+            static_cast<long long>(height) * width, static_cast<int>(width), static_cast<int>(P), static_cast<int>(output_w),
+            static_cast<int>(stride_h), static_cast<int>(stride_w));
+        g_launches.fetch_add(1);
+        CUDA_TRY(cudaGetLastError());
+        q.M = static_cast<long long>(batches) * P;
+        q.N = static_cast<long long>(num_kernels);
+        q.K = static_cast<long long>(channels);
+        q.a.base = pixel_ws;
+        q.a.k_major = 1;
+        q.a.ld = static_cast<long long>(channels);
+        q.b.base = static_cast<const char*>(w);
+        q.b.k_major = 1;
+        q.b.ld = static_cast<long long>(channels);
+        q.d = static_cast<char*>(y);
+        q.ldd = P;
+        q.bias = static_cast<const char*>(bias);
+        q.out_nchw = 1;
+        q.g.P = static_cast<int>(P);
+        q.g.out_img_stride = static_cast<long long>(num_kernels) * P;
+        q.pack_ws = nullptr;
+        q.pack_ws_bytes = 0;
+        rc = split_bank(q, *st, align256(pixel_ws + pixel_bytes), ws_end, true,
+                        static_cast<cudaStream_t>(stream));
+        if (rc != kSuccess) return rc;
+        return launch(q, static_cast<cudaStream_t>(stream), st);
     }
 
     q.M = static_cast<long long>(batches) * P;  // global output pixel index

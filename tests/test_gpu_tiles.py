@@ -334,3 +334,38 @@ def test_copied_fp32_operands_keep_all_but_the_last_bit(lib, ta, tb):
         got = tensor.matmul(A.t() if ta else A, B.t() if tb else B, torch.empty(n, n, device="cuda"))
         want = M.t() if (ta if first else tb) else M
         assert bool(((got.double() - want.double()).abs() <= 2.0 ** -23 * want.double().abs()).all())
+
+
+@pytest.mark.parametrize("scratch", [True, False], ids=["scratch", "no scratch"])
+@pytest.mark.parametrize("n,c,h,w,k,stride", [
+    (150, 4, 4, 4, 8, 1),       # gathered: little but output to write
+    (140, 4, 4, 4, 8, 1),       # ... all tiles at once: a product per image
+    (160, 8, 4, 4, 8, 1),       # an eighth of the rows in use: copied
+    (200, 12, 10, 10, 20, 1),   # three quarters and a bit: a product per image
+    (200, 12, 8, 11, 16, 1),    # less: copied
+    (3, 100, 7, 9, 132, 1),     # odd planes
+    (5, 36, 9, 8, 260, 2),      # stride 2
+    (110, 264, 13, 13, 8, 1),   # gathered, nine k-blocks: a second chunk of one
+    (98, 512, 14, 14, 24, 1),   # a product per image, two waves of tiles: split filters
+    (300, 40, 9, 9, 68, 1),     # copied, two waves of tiles: split filters
+])
+def test_pointwise_fp32_convolutions_on_every_route(lib, n, c, h, w, k, stride, scratch):
+    """Each kernel that a 1x1 filter may go to, with the scratch it asks for and without any; bias, residual, ReLU."""
+    from dlf_b200 import gdnn
+    rng = np.random.default_rng(n + c)
+    f = gdnn.Filter2D((n, c, h, w), (k, c, 1, 1)).strides(stride, stride)
+    X, W = rng.normal(size=(n, c, h, w)).astype(np.float32), (rng.normal(size=(k, c, 1, 1)) / np.sqrt(c)).astype(np.float32)
+    b, R = rng.normal(size=k).astype(np.float32), rng.normal(size=f.output_shape()).astype(np.float32)
+    x, wt, bt, r = (torch.from_numpy(t).cuda() for t in (X, W, b, R))
+    Y = torch.full(f.output_shape(), float("nan"), device="cuda")
+    if scratch:
+        gdnn.conv2d_filter(x, wt, Y, f, bias=bt, residual=r, activation="relu")
+    else:
+        rc = lib.lib().dlf_b200_conv2d_fused(
+            32, n, c, h, w, f.output_h, f.output_w, k, 1, 1, 1, 0, 0, 0, 0, stride, stride, 1, 1, x.data_ptr(), wt.data_ptr(),
+            bt.data_ptr(), r.data_ptr(), 1, Y.data_ptr(), None, 0, torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+    want = np.einsum("oc,nchw->nohw", W[:, :, 0, 0].astype(np.float64), X[:, :, ::stride, ::stride].astype(np.float64))
+    want = np.maximum(want + b[None, :, None, None] + R, 0.0)
+    # chunks of 256 k on every route: 1.8e-6 of the sums (in one chunk, 512 k: 3.6e-6)
+    assert rel_fro(Y.cpu().numpy(), want) <= 2.4e-6

@@ -169,3 +169,25 @@ def test_dependents_are_launched_by_the_warp_that_holds_the_tensor_memory():
             assert "}" not in body[allocated:at], "%s: another warp may start the dependents first" % name
             checked.append(name)
     assert checked == ["contraction_kernel", "contraction_f32_kernel", "contraction_split_kernel"]
+
+
+def _conv_scratch(L, batches, channels, height, width, out, kernels, k=1):
+    return L.dlf_b200_conv2d_workspace_bytes(32, batches, channels, height, width, out[0], out[1], kernels, 1, k, k)
+
+
+def test_pointwise_fp32_convolutions_ask_for_a_copy_of_their_pixels_only_where_they_are_copied(built_lib):
+    """The scratch beyond the packed filters (which a 3 x 3 filter of the same channels bounds from above)."""
+    L = built_lib
+    def bank(channels, kernels):
+        return _conv_scratch(L, 1, channels, 8, 8, (8, 8), kernels, 3)
+
+    # planes the tensor maps take as they are, tiles well filled or few
+    assert _conv_scratch(L, 256, 256, 56, 56, (56, 56), 64) <= bank(256, 64)
+    assert _conv_scratch(L, 8, 64, 8, 8, (8, 8), 64) <= bank(64, 64)
+    # stride 2: the kept pixels, a quarter of the input
+    kept = 8 * 28 * 28 * 256 * 4
+    assert kept <= _conv_scratch(L, 8, 256, 56, 56, (28, 28), 512) <= kept + bank(256, 512)
+    # many pixels and few filters: gathered; padded, or with channels that are no whole 16 bytes: always
+    assert _conv_scratch(L, 151, 200, 56, 56, (28, 28), 16) <= bank(200, 16)
+    assert _conv_scratch(L, 8, 256, 56, 56, (58, 58), 512) <= bank(256, 512)
+    assert _conv_scratch(L, 8, 255, 56, 56, (28, 28), 512) <= bank(255, 512)
