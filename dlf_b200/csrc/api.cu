@@ -70,6 +70,7 @@ struct DeviceState {
     int static_smem_small = 0;
     int static_smem_halo = 0;
     bool split_ready = false;   // contraction_split_kernel is set up
+    bool trsm_ready = false;    // the instantiations of l3_trsm_kernel have their largest shared memory
     int static_smem_f32 = -1;   // contraction_f32_kernel; -1: not set up on this path
     int max_f32_clusters[9] = {0};  // co-resident clusters of [size] CTAs that share a tile's k-blocks
     int max_pair_clusters = 0;  // co-resident CTA pairs of the pair kernel (0 = not usable)
@@ -1651,15 +1652,39 @@ int l3_expand_any(int fmt, void* dst, const void* src, size_t ld, size_t n, bool
 
 namespace {
 
+// An instantiation's limit on shared memory is the kernel's, not a launch's: it is set once, to the most that any order
+// needs (a limit set by each launch to its own need would be lowered by another thread's before the launch).
+template <typename T, bool EQC, int C>
+cudaError_t trsm_limit() {
+    return cudaFuncSetAttribute(l3_trsm_kernel<T, EQC, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(trsm_smem_bytes(kTrsmOrder, C, EQC)));
+}
+
+template <typename T, bool EQC>
+int trsm_limits() {
+    CUDA_TRY((trsm_limit<T, EQC, 4>()));
+    CUDA_TRY((trsm_limit<T, EQC, 8>()));
+    CUDA_TRY((trsm_limit<T, EQC, 16>()));
+    CUDA_TRY((trsm_limit<T, EQC, 24>()));
+    return kSuccess;
+}
+
+int ensure_trsm(DeviceState& st) {
+    std::lock_guard<std::mutex> lock(g_mu);
+    if (st.trsm_ready) return kSuccess;
+    for (int rc : {trsm_limits<float, true>(), trsm_limits<float, false>(), trsm_limits<__half, true>(), trsm_limits<__half, false>(),
+                   trsm_limits<__nv_bfloat16, true>(), trsm_limits<__nv_bfloat16, false>()})
+        if (rc != kSuccess) return rc;
+    st.trsm_ready = true;
+    return kSuccess;
+}
+
 // Systems per CTA of a triangular solve: the fewest that let all CTAs run at once (a step of the chain takes
 // warp 0 as long for 4 systems as for 24, the other warps' part grows with them), 24 when that is not to be had.
 template <typename T, bool EQC, int C>
 int trsm_launch(const void* base, long long se, long long sv, bool unit, size_t q, void* b, long long bu, long long bs,
                 size_t nsys, float alpha, cudaStream_t s) {
-    const size_t smem = trsm_smem_bytes(static_cast<int>(q), C, EQC);
-    auto kernel = l3_trsm_kernel<T, EQC, C>;
-    CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    kernel<<<static_cast<unsigned>((nsys + C - 1) / C), kTrsmThreads, smem, s>>>(
+    l3_trsm_kernel<T, EQC, C><<<static_cast<unsigned>((nsys + C - 1) / C), kTrsmThreads, trsm_smem_bytes(static_cast<int>(q), C, EQC), s>>>(
         static_cast<const T*>(base), se, sv, unit ? 1 : 0, static_cast<int>(q), static_cast<T*>(b), bu, bs,
         static_cast<int>(nsys), alpha);
     g_launches.fetch_add(1);
@@ -2930,6 +2955,10 @@ int dlf_b200_trsm(int dtype, int layout, int side, int triangle, int a_transpose
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     StreamDevice sd(s);
     if (sd.rc != kSuccess) return sd.rc;
+    DeviceState* st = nullptr;
+    rc = ensure_device(&st);
+    if (rc == kSuccess) rc = ensure_trsm(*st);
+    if (rc != kSuccess) return rc;
     clear_stale_error();
     const bool trans = a_transpose != DLF_B200_NO_TRANS;
     const bool lower = triangle == kLower;

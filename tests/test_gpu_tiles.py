@@ -369,3 +369,45 @@ def test_pointwise_fp32_convolutions_on_every_route(lib, n, c, h, w, k, stride, 
     want = np.maximum(want + b[None, :, None, None] + R, 0.0)
     # chunks of 256 k on every route: 1.8e-6 of the sums (in one chunk, 512 k: 3.6e-6)
     assert rel_fro(Y.cpu().numpy(), want) <= 2.4e-6
+
+
+def test_triangular_solves_of_different_orders_from_two_threads(lib):
+    """Solves of order 1024 on one thread's stream and of order 48 on another's: the same kernel with much and with
+    little shared memory. Every call is accepted, and the last results are right."""
+    import ctypes
+    import threading
+    from dlf_b200 import gblas as gb
+    one = ctypes.c_float(1.0)
+    problems, failures = [], []
+    for q in (1024, 48):
+        g = torch.Generator(device="cuda").manual_seed(q)
+        T = torch.randn(q, q, generator=g, device="cuda") * (0.5 / q ** 0.5)
+        T.diagonal().abs_().add_(1.0)
+        problems.append((q, T, torch.randn(q, 64, generator=g, device="cuda")))
+    torch.cuda.synchronize()
+
+    def work(q, T, B):
+        stream = torch.cuda.Stream()
+        X = B.clone()
+        torch.cuda.synchronize()
+        args = [32, gb.Layout.RowMajor, gb.Side.Left, gb.Triangle.Lower, gb.Transpose.NoTrans, gb.Diagonal.NonUnit, q, 64,
+                ctypes.byref(one), T.data_ptr(), q, X.data_ptr(), 64, None, 0, stream.cuda_stream]
+        trsm = lib.lib().dlf_b200_trsm
+        for _ in range(3000):
+            rc = trsm(*args)
+            if rc != 0:
+                failures.append((q, rc))
+        with torch.cuda.stream(stream):
+            X.copy_(B)
+            assert trsm(*args) == 0
+        stream.synchronize()
+        want = torch.linalg.solve_triangular(torch.tril(T).double(), B.double(), upper=False)
+        if rel_fro(X.cpu().numpy(), want.cpu().numpy()) > FP32_TOL:
+            failures.append((q, "result"))
+
+    threads = [threading.Thread(target=work, args=p) for p in problems]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures
