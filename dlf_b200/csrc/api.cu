@@ -1654,10 +1654,10 @@ namespace {
 
 // An instantiation's limit on shared memory is the kernel's, not a launch's: it is set once, to the most that any order
 // needs (a limit set by each launch to its own need would be lowered by another thread's before the launch).
-template <typename T, bool EQC, int C>
+template <typename T, bool EQC, int C, int THREADS = kTrsmThreads>
 cudaError_t trsm_limit() {
-    return cudaFuncSetAttribute(l3_trsm_kernel<T, EQC, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(trsm_smem_bytes(kTrsmOrder, C, EQC)));
+    return cudaFuncSetAttribute(l3_trsm_kernel<T, EQC, C, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(trsm_smem_bytes(kTrsmOrder, C, EQC, THREADS)));
 }
 
 template <typename T, bool EQC>
@@ -1666,6 +1666,8 @@ int trsm_limits() {
     CUDA_TRY((trsm_limit<T, EQC, 8>()));
     CUDA_TRY((trsm_limit<T, EQC, 16>()));
     CUDA_TRY((trsm_limit<T, EQC, 24>()));
+    CUDA_TRY((trsm_limit<T, EQC, 24, 256>()));
+    CUDA_TRY((trsm_limit<T, EQC, 24, 128>()));
     return kSuccess;
 }
 
@@ -1681,10 +1683,10 @@ int ensure_trsm(DeviceState& st) {
 
 // Systems per CTA of a triangular solve: the fewest that let all CTAs run at once (a step of the chain takes
 // warp 0 as long for 4 systems as for 24, the other warps' part grows with them), 24 when that is not to be had.
-template <typename T, bool EQC, int C>
+template <typename T, bool EQC, int C, int THREADS = kTrsmThreads>
 int trsm_launch(const void* base, long long se, long long sv, bool unit, size_t q, void* b, long long bu, long long bs,
                 size_t nsys, float alpha, cudaStream_t s) {
-    l3_trsm_kernel<T, EQC, C><<<static_cast<unsigned>((nsys + C - 1) / C), kTrsmThreads, trsm_smem_bytes(static_cast<int>(q), C, EQC), s>>>(
+    l3_trsm_kernel<T, EQC, C, THREADS><<<static_cast<unsigned>((nsys + C - 1) / C), THREADS, trsm_smem_bytes(static_cast<int>(q), C, EQC, THREADS), s>>>(
         static_cast<const T*>(base), se, sv, unit ? 1 : 0, static_cast<int>(q), static_cast<T*>(b), bu, bs,
         static_cast<int>(nsys), alpha);
     g_launches.fetch_add(1);
@@ -1692,28 +1694,46 @@ int trsm_launch(const void* base, long long se, long long sv, bool unit, size_t 
     return kSuccess;
 }
 
+// Systems per CTA of a triangular solve: the fewest that let all CTAs run at once (a step of the chain takes
+// warp 0 little longer for 24 systems than for 4, the other warps' part grows with them), 24 when that is not to be had.
+// Then it is throughput that counts, and short systems leave most of a CTA's 13 row warps without equations: with fewer
+// warps a CTA, more CTAs are on an SM (fp32, 40000 systems: order 64 83 us with 512 threads, 33 with 128; order 128 175 and 82;
+// order 256 419, 287 with 256 threads, 265 with 128, and at 7104 systems 82, 51 and 82).
+// Few unknowns of many systems go to l3_trsm_small_kernel, a thread per system, from 25 q^2 systems on (order 8:
+// 2500 systems 3.6 and 3.3 us, 40000 34 and 3.3; order 32: 10000 6.1 and 11.6 us, 40000 17.8 and 13.9).
 template <typename T, bool EQC>
-int trsm_columns(const void* base, long long se, long long sv, bool unit, size_t q, void* b, long long bu, long long bs,
+int trsm_columns(int num_sms, const void* base, long long se, long long sv, bool unit, size_t q, void* b, long long bu, long long bs,
                  size_t nsys, float alpha, cudaStream_t s) {
-    if (nsys <= 4 * 148) return trsm_launch<T, EQC, 4>(base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
-    if (nsys <= 8 * 148) return trsm_launch<T, EQC, 8>(base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
-    if (nsys <= 16 * 148) return trsm_launch<T, EQC, 16>(base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
-    return trsm_launch<T, EQC, 24>(base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
+    const size_t sms = static_cast<size_t>(num_sms);
+    if (q <= kTrsmSmall && nsys >= 25 * q * q) {
+        const auto kernel = q <= 32 ? l3_trsm_small_kernel<T, 32> : l3_trsm_small_kernel<T, 64>;
+        kernel<<<static_cast<unsigned>((nsys + kTrsmSmallThreads - 1) / kTrsmSmallThreads), kTrsmSmallThreads, 0, s>>>(
+            static_cast<const T*>(base), se, sv, unit ? 1 : 0, static_cast<int>(q), static_cast<T*>(b), bu, bs, static_cast<int>(nsys), alpha);
+        g_launches.fetch_add(1);
+        CUDA_TRY(cudaGetLastError());
+        return kSuccess;
+    }
+    if (nsys <= 4 * sms) return trsm_launch<T, EQC, 4>(base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
+    if (nsys <= 8 * sms) return trsm_launch<T, EQC, 8>(base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
+    if (nsys <= 16 * sms) return trsm_launch<T, EQC, 16>(base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
+    if (nsys <= 24 * sms || q > 256) return trsm_launch<T, EQC, 24>(base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
+    if (q > 128) return trsm_launch<T, EQC, 24, 256>(base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
+    return trsm_launch<T, EQC, 24, 128>(base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
 }
 
 template <typename T>
-int trsm_any(bool eqc, const void* base, long long se, long long sv, bool unit, size_t q, void* b, long long bu,
+int trsm_any(int num_sms, bool eqc, const void* base, long long se, long long sv, bool unit, size_t q, void* b, long long bu,
              long long bs, size_t nsys, float alpha, cudaStream_t s) {
-    return eqc ? trsm_columns<T, true>(base, se, sv, unit, q, b, bu, bs, nsys, alpha, s)
-               : trsm_columns<T, false>(base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
+    return eqc ? trsm_columns<T, true>(num_sms, base, se, sv, unit, q, b, bu, bs, nsys, alpha, s)
+               : trsm_columns<T, false>(num_sms, base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
 }
 
 // one diagonal block (order q <= kTrsmOrder) of a triangular solve; arguments as of l3_trsm_kernel
-int trsm_block(int fmt, const void* base, long long se, long long sv, bool eqc, bool unit, size_t q, void* b,
+int trsm_block(int num_sms, int fmt, const void* base, long long se, long long sv, bool eqc, bool unit, size_t q, void* b,
                long long bu, long long bs, size_t nsys, float alpha, cudaStream_t s) {
-    if (fmt == FMT_F32) return trsm_any<float>(eqc, base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
-    if (fmt == FMT_F16) return trsm_any<__half>(eqc, base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
-    return trsm_any<__nv_bfloat16>(eqc, base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
+    if (fmt == FMT_F32) return trsm_any<float>(num_sms, eqc, base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
+    if (fmt == FMT_F16) return trsm_any<__half>(num_sms, eqc, base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
+    return trsm_any<__nv_bfloat16>(num_sms, eqc, base, se, sv, unit, q, b, bu, bs, nsys, alpha, s);
 }
 
 // common argument rules of trmm / trsm; on success the call is in row-major form
@@ -2968,8 +2988,18 @@ int dlf_b200_trsm(int dtype, int layout, int side, int triangle, int a_transpose
     char* B = static_cast<char*>(b);
     auto a_at = [&](size_t r, size_t c) { return A + (r * a_ld + c) * es; };
     auto b_at = [&](size_t r, size_t c) { return B + (r * b_ld + c) * es; };
+    // Order of the blocks: as few as kTrsmOrder allows, of about equal order. With very many systems short blocks with
+    // products between them are faster, because a launch's work grows with the square of its order (fp32, 40000 systems
+    // of 1024 unknowns: 3330 us in one launch, 1080 in blocks of 128; 512 unknowns 1030 and 470; fp16 4310 and 1025). But the
+    // products add their own error, and 16-bit unknowns are rounded once more for each (relative error, 20000 systems of 1024:
+    // fp32 5.9e-7 and 6.6e-7, fp16 2.1e-4 and 3.0e-4): only from where blocks of 64 would be as fast as one launch
+    // (fp32, 1024 unknowns: 10000 systems 821 us in one launch, 1015 in blocks of 64; 256 unknowns 115 and 195).
+    const size_t order = side == kLeft ? m : n, nsys = side == kLeft ? n : m;
+    const size_t longest = nsys >= (fmt != FMT_F32 && order > 768 ? 8192u : 16384u) ? 128 : kTrsmOrder;
+    const size_t parts = (order + longest - 1) / longest;
+    const size_t block = ((order + parts - 1) / parts + 31) / 32 * 32;
     // one block: alpha goes in with its right-hand sides; more: the updates need all of B scaled
-    if (al != 1.0f && (side == kLeft ? m : n) > kTrsmOrder) {
+    if (al != 1.0f && parts > 1) {
         const unsigned grid = l3_grid(static_cast<long long>(m) * n);
         if (fmt == FMT_F32) l3_scale_kernel<float><<<grid, 256, 0, s>>>(reinterpret_cast<float*>(B), static_cast<long long>(b_ld), static_cast<int>(m), static_cast<int>(n), al);
         else if (fmt == FMT_F16) l3_scale_kernel<__half><<<grid, 256, 0, s>>>(reinterpret_cast<__half*>(B), static_cast<long long>(b_ld), static_cast<int>(m), static_cast<int>(n), al);
@@ -2977,10 +3007,6 @@ int dlf_b200_trsm(int dtype, int layout, int side, int triangle, int a_transpose
         g_launches.fetch_add(1);
         CUDA_TRY(cudaGetLastError());
     }
-    // order of the blocks: as few as kTrsmOrder allows, of about equal order
-    const size_t order = side == kLeft ? m : n, nsys = side == kLeft ? n : m;
-    const size_t parts = (order + kTrsmOrder - 1) / kTrsmOrder;
-    const size_t block = ((order + parts - 1) / parts + 31) / 32 * 32;
     auto diag_solve = [&](size_t d0, size_t nb, float scale) -> int {
         const bool forward = side == kLeft ? op_lower : !op_lower;
         const long long d1 = static_cast<long long>(forward ? d0 : d0 + nb - 1), dir = forward ? 1 : -1;
@@ -2988,7 +3014,7 @@ int dlf_b200_trsm(int dtype, int layout, int side, int triangle, int a_transpose
         const long long se = dir * (eqc ? 1 : static_cast<long long>(a_ld)), sv = dir * (eqc ? static_cast<long long>(a_ld) : 1);
         const long long bu = side == kLeft ? dir * static_cast<long long>(b_ld) : dir, bs = side == kLeft ? 1 : static_cast<long long>(b_ld);
         char* first = side == kLeft ? b_at(d1, 0) : b_at(0, d1);
-        return trsm_block(fmt, a_at(d1, d1), se, sv, eqc, diagonal == kUnit, nb, first, bu, bs, nsys, scale, s);
+        return trsm_block(st->num_sms, fmt, a_at(d1, d1), se, sv, eqc, diagonal == kUnit, nb, first, bu, bs, nsys, scale, s);
     };
     const int N = DLF_B200_NO_TRANS, T = DLF_B200_TRANS;
     if (side == kLeft) {

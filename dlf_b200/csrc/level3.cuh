@@ -162,14 +162,13 @@ __global__ void __launch_bounds__(256) pad_lines_kernel(const PadLines p) {
 }
 
 constexpr int kTrsmOrder = 1024;   // unknowns one launch solves; longer systems are cut into blocks of this order
-constexpr int kTrsmThreads = 512;
-constexpr int kTrsmRowWarps = kTrsmThreads / 32 - 3;
+constexpr int kTrsmThreads = 512;  // (256 and 128: see trsm_columns in api.cu)
 constexpr int kTrsmTileLd = 36;  // floats between the lines of a staged 32 x 32 tile (16-byte aligned lines)
 constexpr int kTrsmTurn = 64 * 20;  // floats of a row warp's transposition buffer: 64 lines of 16 + 4 or 32 of 32 + 4
 
 // dynamic shared memory of l3_trsm_kernel: the CTA's right-hand sides, then a transposition buffer per row warp
-constexpr size_t trsm_smem_bytes(int q, int columns, bool eq_contiguous) {
-    return static_cast<size_t>((q + 63) / 64 * 64) * columns * 4 + (eq_contiguous ? 0 : kTrsmRowWarps * kTrsmTurn * 4);
+constexpr size_t trsm_smem_bytes(int q, int columns, bool eq_contiguous, int threads) {
+    return static_cast<size_t>((q + 63) / 64 * 64) * columns * 4 + (eq_contiguous ? 0 : (threads / 32 - 3) * kTrsmTurn * 4);
 }
 
 // Substitution, whole: q <= kTrsmOrder unknowns of `nsys` independent systems, C systems per CTA, which stay
@@ -182,18 +181,19 @@ constexpr size_t trsm_smem_bytes(int q, int columns, bool eq_contiguous) {
 // What bounds it is the chain of unknowns, so the block of 32 unknowns at hand is all that warp 0 works on:
 // lane = equation, it takes the newest 32 solved unknowns out of the next 32 equations and solves those, the systems
 // side by side to cover the latency of the shuffles (with many systems lane = system), while warps
-// 1 and 2 fetch the two coefficient tiles warp 0 needs two steps later and the other 13 warps take the newest
+// 1 and 2 fetch the two coefficient tiles warp 0 needs two steps later and the other warps take the newest
 // unknowns out of all later equations (the solved unknowns come from shared memory, 16 bytes a lane,
 // which is what sets their pace), each with its next 32 coefficients already on the way. One barrier
 // per 32 unknowns. A quotient is a product with the reciprocal and one correction step (12 clocks of latency
 // instead of a division's); a block with a result that is not finite is solved again with divisions.
 // Measured (fp32): 1024 unknowns x 512 systems 947 us in 16 launches of one thread per system and 15 products between
 // them, now 93 (equations contiguous) to 119 us (unknowns); 512 x 512 37 to 45, 128 x 512 11 to 13, 48 x 48 6 us.
-template <typename T, bool EQC, int C>
-__global__ void __launch_bounds__(kTrsmThreads, 1)
+template <typename T, bool EQC, int C, int THREADS>
+__global__ void __launch_bounds__(THREADS, 512 / THREADS)
     l3_trsm_kernel(const T* __restrict__ base, long long se, long long sv, int unit, int q, T* __restrict__ b,
                    long long b_unknown, long long b_system, int nsys, float alpha) {
     static_assert(C % 4 == 0 && C <= 32, "a lane of warp 0 solves one system; right-hand sides move as float4");
+    constexpr int kTrsmRowWarps = THREADS / 32 - 3;
     extern __shared__ __align__(16) float trsm_smem[];
     __shared__ __align__(16) float dia[2][32 * kTrsmTileLd];  // [unknown][equation] of the diagonal tile
     __shared__ __align__(16) float sub[2][32 * kTrsmTileLd];  // [unknown][equation] of the tile left of it
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(kTrsmThreads, 1)
     const int total = rows * C;
     const bool across = b_system == 1;
 #pragma unroll 4
-    for (int id = threadIdx.x; id < total; id += kTrsmThreads) {
+    for (int id = threadIdx.x; id < total; id += THREADS) {
         const int p = across ? id / C : id % rows, t = across ? id % C : id / rows;
         R[p * C + t] = p < q && sys0 + t < nsys ? alpha * l3_load(b + p * b_unknown + (sys0 + t) * b_system) : 0.0f;
     }
@@ -499,9 +499,39 @@ __global__ void __launch_bounds__(kTrsmThreads, 1)
         }
     }
 #pragma unroll 4
-    for (int id = threadIdx.x; id < total; id += kTrsmThreads) {
+    for (int id = threadIdx.x; id < total; id += THREADS) {
         const int p = across ? id / C : id % rows, t = across ? id % C : id / rows;
         if (p < q && sys0 + t < nsys) b[p * b_unknown + (sys0 + t) * b_system] = l3_make<T>(R[p * C + t]);
+    }
+}
+
+// The same for few unknowns of many systems, a thread per system; arguments as above. Bound by the chain of q * q / 2
+// multiply-adds with one operand from shared memory each, and from some ten thousand systems on by their traffic.
+// Q: room for that many unknowns, 32 where they fit (20 KB of shared memory a CTA, 48 KB with 64).
+// Measured (fp32, in place): 4 unknowns x 100000 systems 3.3 us (l3_trsm_kernel 80), 32 x 100000 20 (90).
+constexpr int kTrsmSmall = 64;
+constexpr int kTrsmSmallThreads = 128;
+template <typename T, int Q>
+__global__ void __launch_bounds__(kTrsmSmallThreads)
+    l3_trsm_small_kernel(const T* __restrict__ base, long long se, long long sv, int unit, int q, T* __restrict__ b,
+                         long long b_unknown, long long b_system, int nsys, float alpha) {
+    __shared__ float coef[Q][Q];  // [equation][unknown], read as a broadcast
+    __shared__ float xs[Q][kTrsmSmallThreads];
+    for (int id = threadIdx.x; id < q * q; id += kTrsmSmallThreads) {
+        const int eq = id / q, var = id - eq * q;
+        if (var <= eq) coef[eq][var] = var == eq && unit ? 1.0f : l3_load(base + eq * se + var * sv);
+    }
+    __syncthreads();
+    const int t = blockIdx.x * kTrsmSmallThreads + threadIdx.x;
+    if (t >= nsys) return;
+    T* at = b + t * b_system;
+    for (int p = 0; p < q; ++p) xs[p][threadIdx.x] = alpha * l3_load(at + p * b_unknown);
+    for (int p = 0; p < q; ++p) {
+        float acc = xs[p][threadIdx.x];
+        for (int v = 0; v < p; ++v) acc = fmaf(-coef[p][v], xs[v][threadIdx.x], acc);
+        acc /= coef[p][p];
+        xs[p][threadIdx.x] = acc;
+        at[p * b_unknown] = l3_make<T>(acc);
     }
 }
 

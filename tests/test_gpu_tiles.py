@@ -119,7 +119,13 @@ def test_a_products_scratch_covers_its_aligned_copies(lib):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16], ids=["f32", "f16"])
-@pytest.mark.parametrize("q,systems", [(1, 1), (31, 5), (32, 3), (33, 600), (64, 4), (97, 1200), (448, 2400), (1024, 6), (1025, 5)])
+@pytest.mark.parametrize("q,systems", [(1, 1), (31, 5), (32, 3), (33, 600), (64, 4), (97, 1200), (448, 2400), (1024, 6), (1025, 5),
+                                       # a thread per system: from 25 q^2 on, up to 32 and up to 64 unknowns
+                                       (1, 25), (8, 1599), (8, 1600), (32, 25601), (33, 27300),
+                                       # CTAs of 128 and 256 threads: more than 24 systems for each SM
+                                       (33, 3553), (128, 3570), (129, 3553), (256, 3600),
+                                       # many systems: blocks of 128 unknowns
+                                       (128, 16384), (160, 16400), (300, 16384)])
 def test_triangular_solves_at_the_edges_of_their_blocks(lib, dtype, q, systems):
     """l3_trsm_kernel: partly filled blocks of 32 unknowns, each number of systems per CTA, both contiguous
     directions, both substitution orders, the largest order of one launch and one more."""
@@ -383,13 +389,12 @@ def test_triangular_solves_of_different_orders_from_two_threads(lib):
         g = torch.Generator(device="cuda").manual_seed(q)
         T = torch.randn(q, q, generator=g, device="cuda") * (0.5 / q ** 0.5)
         T.diagonal().abs_().add_(1.0)
-        problems.append((q, T, torch.randn(q, 64, generator=g, device="cuda")))
+        B = torch.randn(q, 64, generator=g, device="cuda")
+        want = torch.linalg.solve_triangular(torch.tril(T).double(), B.double(), upper=False).cpu().numpy()
+        problems.append((q, T, B, B.clone(), torch.cuda.Stream(), want))
     torch.cuda.synchronize()
 
-    def work(q, T, B):
-        stream = torch.cuda.Stream()
-        X = B.clone()
-        torch.cuda.synchronize()
+    def work(q, T, B, X, stream, want):
         args = [32, gb.Layout.RowMajor, gb.Side.Left, gb.Triangle.Lower, gb.Transpose.NoTrans, gb.Diagonal.NonUnit, q, 64,
                 ctypes.byref(one), T.data_ptr(), q, X.data_ptr(), 64, None, 0, stream.cuda_stream]
         trsm = lib.lib().dlf_b200_trsm
@@ -399,11 +404,8 @@ def test_triangular_solves_of_different_orders_from_two_threads(lib):
                 failures.append((q, rc))
         with torch.cuda.stream(stream):
             X.copy_(B)
-            assert trsm(*args) == 0
+            failures.extend((q, rc) for rc in [trsm(*args)] if rc != 0)
         stream.synchronize()
-        want = torch.linalg.solve_triangular(torch.tril(T).double(), B.double(), upper=False)
-        if rel_fro(X.cpu().numpy(), want.cpu().numpy()) > FP32_TOL:
-            failures.append((q, "result"))
 
     threads = [threading.Thread(target=work, args=p) for p in problems]
     for t in threads:
@@ -411,3 +413,5 @@ def test_triangular_solves_of_different_orders_from_two_threads(lib):
     for t in threads:
         t.join()
     assert not failures
+    for q, T, B, X, stream, want in problems:
+        assert rel_fro(X.cpu().numpy(), want) <= FP32_TOL
