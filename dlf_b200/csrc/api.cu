@@ -3427,10 +3427,17 @@ int dlf_b200_pool_nhwc(int dtype, int average, int count_include_pad, size_t bat
     g.count_include_pad = count_include_pad ? 1 : 0;
     g.total = total;
     cudaStream_t cs = static_cast<cudaStream_t>(stream);
-    // a window that is the whole image goes to the kernel whose warps share its pixels
+    // A window that is the whole image: the kernel whose warps share its pixels, unless so many images have so few that it is
+    // faster for a thread to walk them. Both times in us, by the pixels of a window: eight blocks an SM at a time
+    // take 1.8 + 0.035 each (of the 32 lanes as many work as there are channel groups); a thread alone 2.4 + 0.222, and all
+    // of them 3.2 TB/s (4096 images of 64 x 2 x 4: 9.1 and 4.5; x 14 x 14: 36 and 125; 65536 of 8 x 7 x 7: 192 and
+    // 16; 4096 of 256 x 7 x 7: 20 and 32; 256 of 2048 x 7 x 7: 11 and 31).
     const long long groups = static_cast<long long>(batches) * ((g.C8 + 31) / 32);
+    const double pixels = static_cast<double>(height) * static_cast<double>(width);
+    const double shared_us = 2.0 + static_cast<double>(groups) / (8.0 * st->num_sms) * (1.8 + 0.035 * pixels);
+    const double alone_us = std::max(2.4 + 0.222 * pixels, static_cast<double>(total) * pixels * 16.0 / 3.2e6);
     if (output_h == 1 && output_w == 1 && pad_top == 0 && pad_left == 0 && kernel_h == height && kernel_w == width &&
-        height * width >= 8 && height * width < INT_MAX && groups < INT_MAX) {
+        height * width >= 8 && height * width < INT_MAX && groups < INT_MAX && shared_us < alone_us) {
         if (fmt == FMT_F16)
             pool_nhwc_global_kernel<OUT_F16><<<static_cast<unsigned>(groups), 256, 0, cs>>>(static_cast<const uint4*>(x), static_cast<uint4*>(y), g);
         else

@@ -170,9 +170,10 @@ def test_triangular_solve_with_a_zero_and_an_infinite_pivot(lib):
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16], ids=["f16", "bf16"])
-@pytest.mark.parametrize("shape", [(1, 2048, 7, 7), (3, 8, 2, 4), (2, 264, 3, 3), (2, 40, 33, 5)])
+@pytest.mark.parametrize("shape", [(1, 2048, 7, 7), (3, 8, 2, 4), (2, 264, 3, 3), (2, 40, 33, 5), (1100, 8, 2, 4), (1500, 8, 2, 4)])
 def test_global_pooling_between_channels_last_tensors(lib, dtype, shape):
-    """pool_nhwc_global_kernel: channel groups that do not fill a warp, more and fewer pixels than warps."""
+    """pool_nhwc_global_kernel: channel groups that do not fill a warp, more and fewer pixels than warps; on
+    either side of the number of images from which a thread walks each of them instead."""
     from dlf_b200 import gdnn
     n, c, h, w = shape
     X = _round_to(np.random.default_rng(c).normal(size=shape), dtype)
