@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <atomic>
 #include <climits>
+#include <cmath>
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
@@ -1086,7 +1087,10 @@ int launch(const Problem& q_in, cudaStream_t stream, DeviceState* preset = nullp
     if (q_in.es == 2 && (q_in.out_nchw == 5 || (q_in.out_nchw == 0 && q_in.a_cl == 0 && q_in.bias == nullptr && q_in.resid == nullptr))) {
         const Problem qs = q_in.out_nchw == 5 ? q_in : exchanged(q_in);
         const int ctas = split_ctas(*st, qs);
-        if (ctas > 0) {
+        // (One CTA a tile is what contraction_kernel is as well, with its epilogue beside the next tile's loads: 1024 x 1024 x 256
+        // 4.9 us, 5.9 here; channels-last 3x3 256 -> 256 on 16 images of 14 x 14 12.6 and 14.4. It needs rows that
+        // fill its lanes, though: 72 x 1024 x 256 5.1 us, 4.5 here.)
+        if (ctas > 1 || (ctas == 1 && q_in.out_nchw == 0 && qs.M < kBM)) {
             rc = launch_split(*st, qs, ctas, stream);
             if (rc != kNotImplemented) return rc;  // else: window corners outside the im2col map's range
         }
@@ -1564,6 +1568,23 @@ size_t splitk_slices(const Problem& q, int num_sms) {
     return best;
 }
 
+// Whether a product that could be cut into `slices` is faster in one launch. Where the tensor maps take its operands
+// that launch has a CTA or a cluster of CTAs per tile, and a cluster shares its tile's K range out. A cluster has 8 CTAs at
+// most, so 16 tiles and fewer fill more SMs as slices. fp32: always beyond that. 16 bit: by the k-blocks that a
+// CTA then walks, 0.27 us each, against the second launch, the partial products' way through memory and the k-blocks
+// of a slice (fp16, us in one launch and in slices: 1024 x 1024 x 2048 13.6 and 19.1, x 8192 40.2 and 34.0;
+// 640 x 1024 x 2048 13.0 and 15.4, x 8192 39.1 and 22.8; 16 x 4096 x 1024 7.8 and 8.9, x 8192 22.6 and 16.6).
+bool one_launch(const DeviceState& st, const Problem& q, long long slices) {
+    if (((q.M + kBM - 1) / kBM) * ((q.N + 127) / 128) <= 16) return false;
+    if (q.es == 4) return f32_tma_ok(st, q);
+    const int ctas = split_ctas(st, exchanged(q));
+    if (ctas == 0) return false;
+    const double num_kb = static_cast<double>((q.K + 63) / 64);
+    const double whole_us = (q.N < kBM ? 6.2 : 4.2) + 0.27 * std::ceil(num_kb / ctas);  // (few rows: 2 us more)
+    const double sliced_us = 7.5 + 5.5e-6 * static_cast<double>(q.M) * static_cast<double>(q.N) + 0.28 * num_kb / static_cast<double>(slices);
+    return whole_us <= sliced_us;
+}
+
 int launch_splitk(const Problem& q, size_t slices, void* workspace, cudaStream_t stream, DeviceState* st) {
     Problem r = q;
     const long long ks = q.K / static_cast<long long>(slices);
@@ -1889,10 +1910,7 @@ int dlf_b200_gemm_ex(int dtype, int layout, int trans_a, int trans_b, size_t m, 
             workspace_bytes -= need;
         }
     }
-    // A product with few tiles whose operands the tensor maps take can share a tile's K range out inside one launch,
-    // over the CTAs of a cluster. A cluster has 8 at most: 16 tiles and fewer fill more SMs as slices of a launch.
-    const bool in_cluster = ((q.M + kBM - 1) / kBM) * ((q.N + 127) / 128) > 16 && (split_ctas(*st, exchanged(q)) > 0 || f32_tma_ok(*st, q));
-    if (workspace != nullptr && !(g_force_generic.load() & 0x20000000) && !in_cluster) {
+    if (workspace != nullptr && !(g_force_generic.load() & 0x20000000)) {
         char* ws = align256(workspace);
         const size_t slack = static_cast<size_t>(ws - static_cast<char*>(workspace));
         size_t slices = splitk_slices(q, st->num_sms);
@@ -1903,7 +1921,7 @@ int dlf_b200_gemm_ex(int dtype, int layout, int trans_a, int trans_b, size_t m, 
                                         (q.K / static_cast<long long>(slices) * (q.a.k_major ? 1 : q.a.ld) * q.es) % 16 == 0 &&
                                         (q.K / static_cast<long long>(slices) * (q.b.k_major ? 1 : q.b.ld) * q.es) % 16 == 0);
         while (slices > 1 && workspace_bytes < slack + slices * q.M * q.N * sizeof(float)) slices /= 2;
-        if (slices > 1 && fast) return launch_splitk(q, slices, ws, s, st);
+        if (slices > 1 && fast && !one_launch(*st, q, static_cast<long long>(slices))) return launch_splitk(q, slices, ws, s, st);
     }
     return launch(q, s, st);
 }
@@ -3360,7 +3378,7 @@ int dlf_b200_conv2d_nhwc(int dtype, size_t batches, size_t channels, size_t heig
         // 256 -> 64 1x1: 81 -> 108 us), nor for 1x1 filters (512 -> 128 at 28x28: 48 -> 50 us).
         // Bit 28 of the tile-width word: never.
         // (Too few pixels to fill the GPU with tiles: contraction_split_kernel takes the form as it is.)
-        if (num_kernels > 64 && num_kernels <= 128 && taps > 1 && !((g_force_bn.load() >> 16) & 4096) && split_ctas(*st, q) == 0) {
+        if (num_kernels > 64 && num_kernels <= 128 && taps > 1 && !((g_force_bn.load() >> 16) & 4096) && split_ctas(*st, q) <= 1) {
             std::swap(q.a, q.b);
             q.M = static_cast<long long>(num_kernels);
             q.N = static_cast<long long>(batches) * P;

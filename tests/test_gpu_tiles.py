@@ -416,3 +416,39 @@ def test_triangular_solves_of_different_orders_from_two_threads(lib):
     assert not failures
     for q, T, B, X, stream, want in problems:
         assert rel_fro(X.cpu().numpy(), want) <= FP32_TOL
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16], ids=["f16", "bf16"])
+@pytest.mark.parametrize("m,n,k", [
+    (136, 2304, 2048),   # 36 tiles of 128 x 128: a cluster of two for each tile of 128 x 64
+    (640, 1024, 1024),   # 40: one CTA a tile
+    (640, 1024, 8192),   # ... and so many k-blocks that they are cut into slices
+    (16, 4096, 8192),    # 32 tiles of few rows, sliced
+    (72, 1024, 256),     # one CTA a tile of the cluster kernel, few rows
+])
+def test_16_bit_products_in_one_launch_or_in_slices(lib, dtype, m, n, k):
+    """Either side of the rule that cuts a product's K range between the CTAs of a cluster or between launches."""
+    from dlf_b200 import tensor
+    g = torch.Generator().manual_seed(k)
+    A, B = (torch.rand(m, k, generator=g) - 0.5).to(dtype).cuda(), (torch.rand(k, n, generator=g) - 0.5).to(dtype).cuda()
+    got = tensor.matmul(A, B, torch.empty(m, n, dtype=dtype, device="cuda"))
+    assert max_rel(got.float().cpu().numpy(), (A.double() @ B.double()).cpu().numpy()) <= HALF_TOL
+
+
+def test_a_forward_of_clusters_and_dependent_launches_repeats_itself(lib):
+    """Partial tiles are added in rank order and dependent launches wait for what they read: the same bits every time."""
+    from dlf_b200 import gdnn
+    g = torch.Generator().manual_seed(2)
+    X = (torch.rand(1, 14, 14, 256, generator=g) - 0.5).half().cuda()
+    f = gdnn.Filter2D((1, 256, 14, 14), (256, 256, 3, 3)).pads(1, 1)
+    W = [gdnn.pack_filters_nhwc(((torch.rand(256, 256, 3, 3, generator=g) - 0.5) / 16).half().cuda()) for _ in range(4)]
+    first = None
+    for _ in range(50):
+        x = X
+        for w in W:
+            y = torch.empty_like(X)
+            gdnn.conv2d_nhwc(x, w, y, f, residual=X, activation="relu")
+            x = y
+        if first is None:
+            first = x
+        assert torch.equal(x, first)
