@@ -605,7 +605,16 @@ int choose_bn_ts(const Problem& q, int num_sms, int max_bn, int a_cols, long lon
 // commit that hands the finished accumulator to the epilogue, with a wait limit of 2^21 clocks
 // (about a millisecond) instead of 2^32. The epilogue's wait then runs out, every role drains,
 // tensor memory is freed and the status word reports the time-out; nothing traps or faults, and
-// the next launch runs normally.
+// the next launch runs normally. (With bit 0x20000000 too, contraction_split_kernel and contraction_f32_kernel do so, which
+// any other bit keeps a product away from.)
+constexpr unsigned kWithholdInClusters = 0x30000000u;
+
+// whether the tuning word leaves the kernels whose tiles a cluster may share in use
+bool cluster_kernels_on() {
+    const unsigned bits = static_cast<unsigned>(g_force_generic.load());
+    return bits == 0 || bits == kWithholdInClusters;
+}
+
 // multiply-shift constants for a divisor (see FastDiv in contraction.cuh); {0, 0} = divide plainly
 FastDiv make_fastdiv(long long d) {
     FastDiv f{0u, 0u};
@@ -861,7 +870,7 @@ cudaError_t launch_dependent(void (*kernel)(Formal...), unsigned grid, unsigned 
 // Whether a problem can go to contraction_f32_kernel: both operands through tensor maps, one alpha and beta, plain
 // output. Any tuning bit of the operand paths keeps the general fp32 kernel, which those bits belong to.
 bool f32_tma_ok(const DeviceState& st, const Problem& q) {
-    return q.es == 4 && st.static_smem_f32 >= 0 && g_force_generic.load() == 0 && q.a_cl == 0 && (q.out_nchw == 0 || q.out_nchw == 1) &&
+    return q.es == 4 && st.static_smem_f32 >= 0 && cluster_kernels_on() && q.a_cl == 0 && (q.out_nchw == 0 || q.out_nchw == 1) &&
            !q.a.im2col && !q.rc_kw && q.a_offs == nullptr && q.b_offs == nullptr && q.d_offs == nullptr &&
            q.alphas == nullptr && q.betas == nullptr && q.a_idx == nullptr && q.b_idx == nullptr && q.d_idx == nullptr &&
            (q.bias == nullptr || (!q.bias_rows && q.bias_stride == 0 && q.alpha == 1.0f)) && tma_ok(q.a, q.es, q.M, q.K, q.batch) && tma_ok(q.b, q.es, q.N, q.K, q.batch);
@@ -985,7 +994,7 @@ int launch_f32(const DeviceState& st, const Problem& q, cudaStream_t stream) {
 // CTAs per tile of contraction_split_kernel for a problem in its form (rows of D contiguous along q.N), or 0 when
 // the problem is not one for it: too many tiles to run at once, or an operand or output it cannot address.
 int split_ctas(const DeviceState& st, const Problem& q) {
-    if (q.es != 2 || !st.split_ready || g_force_generic.load() != 0 || g_force_bn.load() != 0 || q.d_f32 || q.cl_swap ||
+    if (q.es != 2 || !st.split_ready || !cluster_kernels_on() || g_force_bn.load() != 0 || q.d_f32 || q.cl_swap ||
         q.a.im2col || q.rc_kw || q.a_offs != nullptr || q.b_offs != nullptr || q.d_offs != nullptr || q.alphas != nullptr ||
         q.betas != nullptr || q.a_idx != nullptr || q.b_idx != nullptr || q.d_idx != nullptr || q.bias_rows || q.a_cl > 1)
         return 0;

@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(kF32Threads, 1)
                             sph ^= 1u;
                         }
                     }
-                    if (ok && ptx::elect_one()) ptx::umma_commit(ptx::smem_u32(&tfull_bar[buf]));
+                    if (ok && !p.skip_tile_commit && ptx::elect_one()) ptx::umma_commit(ptx::smem_u32(&tfull_bar[buf]));
                     __syncwarp();
                     buf ^= 1u;
                     if (buf == 0) tphase ^= 1u;

@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
                 ph ^= 1u;
             }
         }
-        if (ok && ptx::elect_one()) ptx::umma_commit(ptx::smem_u32(&done_bar));
+        if (ok && !p.skip_tile_commit && ptx::elect_one()) ptx::umma_commit(ptx::smem_u32(&done_bar));
         __syncwarp();
     } else if (warp < 4) {
         // ------------------------------------------------------------ accumulator -> partial tile

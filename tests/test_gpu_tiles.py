@@ -107,15 +107,60 @@ def test_products_of_operands_off_16_byte_boundaries(lib, dtype, m, n, k):
 
 
 def test_a_products_scratch_covers_its_aligned_copies(lib):
-    """dlf_b200_gemm_scratch_bytes is dlf_b200_gemm_workspace_bytes plus the copies a call needs; without
-    scratch the same call runs in one launch."""
+    """dlf_b200_gemm_scratch_bytes is dlf_b200_gemm_workspace_bytes plus the copies a call needs. With that much the copies
+    are a launch of their own; with too little for them, or nothing, the same call runs in one launch."""
+    import ctypes
     L = lib.lib()
-    a = torch.zeros(200 * 515, dtype=torch.float16, device="cuda")
-    common = (16, 101, 111, 111, 150, 160, 512)
-    base = L.dlf_b200_gemm_workspace_bytes(16, 150, 160, 512)
-    assert L.dlf_b200_gemm_scratch_bytes(*common, a.data_ptr(), 512, a.data_ptr(), 160) == base
-    more = L.dlf_b200_gemm_scratch_bytes(*common, a.data_ptr() + 2, 512, a.data_ptr(), 160)
-    assert more >= base + 150 * 512 * 2
+    m, n, k = 150, 160, 512
+    g = torch.Generator().manual_seed(4)
+    a = (torch.rand(m * k + 1, generator=g) - 0.5).half().cuda()
+    b = (torch.rand(k * n, generator=g) - 0.5).half().cuda()
+    common = (16, 101, 111, 111, m, n, k)
+    base = L.dlf_b200_gemm_workspace_bytes(16, m, n, k)
+    assert L.dlf_b200_gemm_scratch_bytes(*common, a.data_ptr(), k, b.data_ptr(), n) == base
+    more = L.dlf_b200_gemm_scratch_bytes(*common, a.data_ptr() + 2, k, b.data_ptr(), n)
+    assert more >= base + m * k * 2
+    want = (a[1:].double().view(m, k) @ b.double().view(k, n)).flatten().cpu().numpy()
+    one, zero = ctypes.c_uint16(0x3C00), ctypes.c_uint16(0)
+    ws = torch.empty(more, dtype=torch.uint8, device="cuda")
+    launches = {}
+    for nbytes in (0, m * k, more):
+        c = torch.zeros(m * n, dtype=torch.float16, device="cuda")
+        before = lib.launch_count()
+        assert L.dlf_b200_gemm_ex(*common, ctypes.byref(one), a.data_ptr() + 2, k, b.data_ptr(), n, ctypes.byref(zero), c.data_ptr(), n,
+                                  ws.data_ptr() if nbytes else None, nbytes, torch.cuda.current_stream().cuda_stream) == 0
+        launches[nbytes] = lib.launch_count() - before
+        assert max_rel(c.float().cpu().numpy(), want) <= HALF_TOL
+    assert launches[0] == launches[m * k] == 1 and launches[more] > 1
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32], ids=["f16", "f32"])
+@pytest.mark.parametrize("k", [128, 2048], ids=["one CTA", "a cluster"])
+def test_waits_that_run_out_in_kernels_whose_tiles_a_cluster_may_share(lib, dtype, k):
+    """The bounded waits of contraction_split_kernel and contraction_f32_kernel, made to run out once: with the test aid
+    0x30000000 a single-tile launch withholds the commit that hands the accumulator on and waits about a millisecond. Every CTA
+    of the cluster leaves, the status reports the time-out once, C keeps its contents, the next call is right."""
+    from dlf_b200 import gblas as gb
+    m, n = 64, 64
+    g = torch.Generator().manual_seed(8)
+    A, B = ((torch.rand(s, generator=g) * 2 - 1).to(dtype).cuda() for s in (m * k, k * n))
+    C = torch.full((m * n,), 5.0, dtype=dtype, device="cuda")
+
+    def product():
+        gb.gemm(gb.Layout.RowMajor, gb.Transpose.NoTrans, gb.Transpose.NoTrans, m, n, k, 1.0, A, 0, k, B, 0, n, 0.0, C, 0, n)
+        torch.cuda.synchronize()
+
+    lib.set_tuning(0, 0x30000000)
+    try:
+        product()
+    finally:
+        lib.set_tuning(0, 0)
+    assert lib.device_status() == 1
+    assert lib.device_status() == 0
+    assert bool((C == 5.0).all())
+    product()
+    ref = (A.double().view(m, k) @ B.double().view(k, n)).flatten().cpu().numpy()
+    assert _close(C.float().cpu().numpy(), ref, dtype)
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16], ids=["f32", "f16"])
@@ -155,18 +200,22 @@ def test_triangular_solves_at_the_edges_of_their_blocks(lib, dtype, q, systems):
                     assert max_rel(g, ref) <= 5e-2, (side, tri, ta)
 
 
-def test_triangular_solve_with_a_zero_and_an_infinite_pivot(lib):
+@pytest.mark.parametrize("systems", [3, 1300, 3600, 40000], ids=["shuffles", "lane per system", "short CTAs", "thread per system"])
+def test_triangular_solve_with_a_zero_and_an_infinite_pivot(lib, systems):
     """What IEEE division gives: x / 0 = inf, 0 / 0 = NaN, x / inf = 0, and nothing spreads backwards."""
     from dlf_b200 import gblas as gb
     n = 40
     T = torch.eye(n, device="cuda")
-    T[5, 5], T[7, 7], T[36, 36] = 0.0, float("inf"), 2.0
-    B = torch.ones(n, 3, device="cuda")
+    T[2, 2], T[5, 5], T[36, 36] = float("inf"), 0.0, 2.0
+    B = torch.ones(n, systems, device="cuda")
     B[5, 1] = 0.0
-    gb.trsm(gb.Layout.RowMajor, gb.Side.Left, gb.Triangle.Lower, gb.Transpose.NoTrans, gb.Diagonal.NonUnit, n, 3, 1.0,
-            T.view(-1), 0, n, B.view(-1), 0, 3)
+    gb.trsm(gb.Layout.RowMajor, gb.Side.Left, gb.Triangle.Lower, gb.Transpose.NoTrans, gb.Diagonal.NonUnit, n, systems, 1.0,
+            T.view(-1), 0, n, B.view(-1), 0, systems)
     got = B.cpu()
-    assert torch.isinf(got[5, 0]) and torch.isnan(got[5, 1]) and bool((got[:5] == 1.0).all())
+    expected = torch.ones(5, systems)
+    expected[2] = 0.0
+    assert torch.equal(got[:5], expected)
+    assert bool(torch.isinf(got[5, [0, 2]]).all()) and bool(torch.isnan(got[5, 1]))
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16], ids=["f16", "bf16"])
