@@ -71,6 +71,7 @@ struct DeviceState {
     int static_smem_small = 0;
     int static_smem_halo = 0;
     bool split_ready = false;   // contraction_split_kernel is set up
+    int max_split_clusters[9] = {0};  // its co-resident clusters of 2, 4, 8 CTAs ([CTAs])
     bool trsm_ready = false;    // the instantiations of l3_trsm_kernel have their largest shared memory
     int static_smem_f32 = -1;   // contraction_f32_kernel; -1: not set up on this path
     int max_f32_clusters[9] = {0};  // co-resident clusters of [size] CTAs that share a tile's k-blocks
@@ -203,6 +204,15 @@ int setup_tma_kernels(DeviceState& st) {
     st.static_smem_f32 = worst;
     for (auto k : {contraction_split_kernel<OUT_F16>, contraction_split_kernel<OUT_BF16>})
         CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, split_smem_bytes(kSplitMaxStages)));
+    cfg.blockDim = dim3(kSplitThreads, 1, 1);
+    cfg.dynamicSmemBytes = static_cast<size_t>(split_smem_bytes(kSplitMaxStages));
+    for (int size = 2; size <= kSplitMaxCtas; size *= 2) {
+        attr.val.clusterDim.x = static_cast<unsigned>(size);
+        cfg.gridDim = dim3(static_cast<unsigned>(size * st.num_sms), 1, 1);
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, contraction_split_kernel<OUT_F16>, &cfg) == cudaSuccess) st.max_split_clusters[size] = n;
+    }
+    (void)cudaGetLastError();
     st.split_ready = true;
     return kSuccess;
 }
@@ -1007,8 +1017,7 @@ int split_ctas(const DeviceState& st, const Problem& q) {
     if (tiles > st.num_sms) return 0;
     const long long num_kb = (q.K + 63) / 64;
     int s = 1;
-    // (GPCs hold whole clusters: 4 and 8 CTAs do not tile all 148 SMs)
-    while (2 * s <= kSplitMaxCtas && tiles * 2 * s <= (2 * s > 2 ? 128 : st.num_sms) && num_kb >= 8 * s) s *= 2;
+    while (2 * s <= kSplitMaxCtas && tiles <= st.max_split_clusters[2 * s] && num_kb >= 8 * s) s *= 2;
     return s;
 }
 
@@ -1327,7 +1336,8 @@ int launch(const Problem& q_in, cudaStream_t stream, DeviceState* preset = nullp
     cfg.dynamicSmemBytes = dyn_smem;
     cfg.stream = stream;
     // Programmatic dependent launch (see launch_split) for convolutions, which follow one another in a network
-    // (forward of 256 images 4092 -> 4063 us), and for products of at most two waves of tiles; longer products gain
+    // (256 x 256 x 14 x 14 3x3 in fp16 with its copies 82.7 -> 78.6 us; the forward of 256 images, layers of 60 us and more,
+    // within its noise), and for products of at most two waves of tiles; longer products gain
     // nothing by it (4096^3 125.1 / 125.9 us, 1024 x (512 x 512 x 64) 131.8 / 133.2 us without / with).
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1521,7 +1531,7 @@ PadPlan pad_plan(const Problem& q) {
 }
 
 // copies the operands the plan names into `ws` and points the problem at the copies
-int pad_operands(Problem& q, const PadPlan& plan, char* ws, cudaStream_t stream) {
+int pad_operands(Problem& q, const PadPlan& plan, int num_sms, char* ws, cudaStream_t stream) {
     PadLines p{};
     int n = 0;
     long long most = 0;
@@ -1546,7 +1556,7 @@ int pad_operands(Problem& q, const PadPlan& plan, char* ws, cudaStream_t stream)
         q.b_lo = p.dst[n - 1] + p.lo[n - 1];
     }
     clear_stale_error();
-    const dim3 grid(static_cast<unsigned>(std::min<long long>((most + 255) / 256, 148 * 8)), static_cast<unsigned>(n));
+    const dim3 grid(static_cast<unsigned>(std::min<long long>((most + 255) / 256, 8ll * num_sms)), static_cast<unsigned>(n));
     if (q.es == 2) pad_lines_kernel<2><<<grid, 256, 0, stream>>>(p);
     else pad_lines_kernel<4><<<grid, 256, 0, stream>>>(p);
     g_launches.fetch_add(1);
@@ -1913,7 +1923,7 @@ int dlf_b200_gemm_ex(int dtype, int layout, int trans_a, int trans_b, size_t m, 
         char* ws = align256(workspace);
         const size_t need = static_cast<size_t>(ws - static_cast<char*>(workspace)) + plan.bytes();
         if (plan.bytes() > 0 && workspace_bytes >= need) {
-            rc = pad_operands(q, plan, ws, s);
+            rc = pad_operands(q, plan, st->num_sms, ws, s);
             if (rc != kSuccess) return rc;
             workspace = ws + plan.bytes();
             workspace_bytes -= need;
