@@ -9,9 +9,9 @@
 // 2^-21 of itself, one of A to 2^-23. Where this kernel stands in for one that rounds both parts of B too - the filters of
 // 1x1 convolutions, B operands off 16-byte boundaries - it does the same: with F32_B_ROUND the converters write hi over
 // the raw tile as well, with F32_B_SPLIT hi and lo are two matrices that a copy has written (pad_lines_kernel) and
-// TMA fetches both. Rounding in the kernel is for launches of one wave of tiles, which another launch would cost more
-// (64 -> 64 channels, 64 images of 8 x 8: 5.8 us truncated, 6.4 rounded here); over many waves the converters are too
-// slow for it (256 -> 256, 64 images of 56 x 56: 150 us truncated, 196 rounded here, 143 from two matrices).
+// TMA fetches both. Rounding in the kernel is for launches that walk a dozen k-blocks in a row or fewer, which another
+// launch would cost more (64 -> 64 channels, 64 images of 8 x 8: 5.8 us truncated, 5.9 rounded here); over more the converters are
+// too slow for it (256 -> 256, 64 images of 56 x 56: 150 us truncated, 196 rounded here, 143 from two matrices).
 // The tensor core truncates when it adds into its accumulator, so it gets chunks of 8 k-blocks; eight
 // epilogue warps add the finished chunks with rounding to nearest, in registers (32 x 32*NB values per warp).
 //
