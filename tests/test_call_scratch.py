@@ -55,7 +55,7 @@ class _Matrix:
 
 
 @pytest.fixture
-def product(monkeypatch):
+def product(monkeypatch, built_lib):  # (a failed call asks the real library for its text)
     def install(**kw):
         library = _Library(**kw)
         monkeypatch.setattr(gb, "lib", lambda: library)
